@@ -6,13 +6,13 @@
  *
  * Single mesh (igab_autotune):
  *   residual       elements per block: tile edge 2 or 4 of the 8-colour schedule
- *   FP64 tangent   FP64 tensor path (mma f64) or FP64 FMA pipe
- *   FP32 tangent   tcgen05 tensor cores (TF32 hi/lo) or FP32 FMA pipe
+ *   FP64 tangent   sum factorisation (mma f64) or the direct form on the FP64 FMA pipe
+ *   FP32 tangent   the same sum factorisation or the direct form on the FP32 FMA pipe
  *   colour order   natural, mirrored or Gray (igab_colour_at), on the sum of the
  *                  kernels chosen above
  * Batch (igab_batch_autotune):
- *   CTAs per SM of the persistent residual and FP64 tangent kernels (1 or as many
- *   as fit; the FP32 kernel runs one CTA per work item), the instance
+ *   CTAs per SM of the persistent residual and tangent kernels (1 or as many
+ *   as fit), the instance
  *   order of the colour-major work list (natural or largest first) and the
  *   colour order.
  * Tile size, CTA count and instance order leave every per-entry summation order
@@ -164,8 +164,8 @@ extern "C" int igab_batch_autotune(igab_batch *b, const double *U_dev, int what,
     IGAB_CUDA_TRY(cudaMalloc(&R.p, (size_t)ndof * sizeof(double)));
     if (what & 14) IGAB_CUDA_TRY(cudaMalloc(&V.p, (size_t)nnz * sizeof(double)));
     int occ[3] = {0, 0, 0};
-    if ((rc = igab_batch_occupancy_res(&occ[0])) || (rc = igab_batch_occupancy_dmma(&occ[1])) ||
-        (rc = igab_batch_occupancy_tc32(&occ[2])))
+    if ((rc = igab_batch_occupancy_res(&occ[0])) || (rc = igab_batch_occupancy_tan(IGAB_PREC_FP64, &occ[1])) ||
+        (rc = igab_batch_occupancy_tan(IGAB_PREC_FP32, &occ[2])))
         return rc;
     int cur[4];
     if ((rc = igab_batch_get_schedule(b, &cur[0], &cur[1], &cur[2], &cur[3]))) return rc;
@@ -179,8 +179,7 @@ extern "C" int igab_batch_autotune(igab_batch *b, const double *U_dev, int what,
         for (int k = 0; k < 3 && !rc; k++) {
             if (!(what & (1 << k))) continue;
             std::vector<int> cands = {0};
-            if (k != 2)   /* the FP32 batch kernel runs one CTA per work item: no CTA count to choose */
-                for (int c = 1; c < occ[k]; c++) cands.push_back(c);
+            for (int c = 1; c < occ[k]; c++) cands.push_back(c);
             double bk = 1e300;
             for (int cand : cands) {
                 int sch[3] = {pick[0], pick[1], pick[2]};

@@ -166,8 +166,7 @@ int grid_of(const igab_batch *b, int what, int *grid)
 {
     int per = 0, rc;
     if (what == 0) rc = igab_batch_occupancy_res(&per);
-    else if (what == 1) rc = igab_batch_occupancy_dmma(&per);
-    else rc = igab_batch_occupancy_tc32(&per);
+    else rc = igab_batch_occupancy_tan(what == 1 ? IGAB_PREC_FP64 : IGAB_PREC_FP32, &per);
     if (rc) return rc;
     if (per < 1) {
         igab_set_error("batch kernel %d does not fit on an SM", what);
@@ -208,9 +207,7 @@ int launch_tangent(igab_batch *b, const double *dU, void *dv, int prec)
     const size_t es = prec == IGAB_PREC_FP64 ? sizeof(double) : sizeof(float);
     IGAB_CUDA_TRY(cudaMemsetAsync(dv, 0, (size_t)b->nnz_off[b->n] * es, b->stream));
     if ((rc = reset_sync(b))) return rc;
-    if (prec == IGAB_PREC_FP64) rc = igab_launch_tan_dmma_batch(dev_view(b), grid, b->stream, dU, (double *)dv);
-    else rc = igab_launch_tan_tc32_batch(dev_view(b), grid, b->stream, dU, (float *)dv);
-    if (rc) return rc;
+    if ((rc = igab_launch_tan_sf_batch(dev_view(b), grid, b->stream, dU, dv, prec))) return rc;
     b->last_launches = 1;
     if (b->nd > 0) {
         if ((rc = igab_launch_tan_dirichlet_batch(dev_view(b), b->nd, b->d_dinst, b->d_drow_l, dv, prec, b->stream)))

@@ -115,8 +115,8 @@ struct igab_ctx {
     int vals_prec = -1;
 
     int tile_res = 2, tile_tan = 2;
-    int tan_kernel = 1;   /* FP64 tangent: 1 tensor-core (mma f64), 0 SIMT */
-    int tan32_kernel = 1; /* FP32 tangent: 1 tcgen05 tensor cores (TF32 hi/lo), 0 SIMT */
+    int tan_kernel = 1;   /* FP64 tangent: 1 sum factorisation (mma f64), 0 direct SIMT form */
+    int tan32_kernel = 1; /* FP32 tangent: 1 the same, FP32 values, 0 direct SIMT form */
     int colour_order = 0; /* igab_colour_order */
     int *d_status = nullptr;   /* device status word: nonzero after a bounded wait gave up */
     int last_launches = 0;
@@ -222,23 +222,20 @@ int igab_launch_csr_cols(igab_ctx *c, int *dcols);
 int igab_launch_check_finite(igab_ctx *c, const void *dev, long n, int prec, int *all_finite);
 int igab_launch_basis_tables(igab_ctx *c, int d, const double *dkv, const double *dgx, const double *dgw);
 int igab_launch_fma_peak(int prec, double *tflops);
-int igab_launch_dmma_peak(double *tflops);   /* igab_tangent_dmma.cu */
+int igab_launch_dmma_peak(double *tflops);   /* igab_probes.cu */
 /* tangent volume kernels over the tiles with x tile coordinate in [tx0, tx1) (tiles of 2 elements) */
-int igab_launch_tan_dmma(igab_ctx *c, const double *dU, double *dv, int tx0, int tx1);
-int igab_launch_tan_tc32(igab_ctx *c, const double *dU, float *dv, int tx0, int tx1);
+int igab_launch_tan_sf(igab_ctx *c, const double *dU, void *dv, int prec, int tx0, int tx1);   /* igab_tangent_sf.cu */
 /* persistent batched launches (igab_batch.cu builds the work list) */
 int igab_launch_res_batch(const igab_batch_dev &B, int grid, cudaStream_t s, const double *dU, double *dR);
-int igab_launch_tan_dmma_batch(const igab_batch_dev &B, int grid, cudaStream_t s, const double *dU, double *dv);
-int igab_launch_tan_tc32_batch(const igab_batch_dev &B, int grid, cudaStream_t s, const double *dU, float *dv);
+int igab_launch_tan_sf_batch(const igab_batch_dev &B, int grid, cudaStream_t s, const double *dU, void *dv, int prec);
 int igab_launch_tan_dirichlet_batch(const igab_batch_dev &B, long nd, const int *dinst, const int *drow, void *dv,
                                     int prec, cudaStream_t s);
 /* R = U - g on a list of (global) Dirichlet rows */
 int igab_launch_res_dirichlet_rows(long nd, const int *drow, const double *dg, const double *dU, double *dR,
                                    cudaStream_t s);
-/* CTAs per SM the persistent kernels can hold (occupancy; the FP32 tangent is capped at 2 by its tensor memory) */
+/* CTAs per SM the persistent kernels can hold */
 int igab_batch_occupancy_res(int *per_sm);
-int igab_batch_occupancy_dmma(int *per_sm);
-int igab_batch_occupancy_tc32(int *per_sm);
+int igab_batch_occupancy_tan(int prec, int *per_sm);
 int igab_launch_tan_getime(igab_ctx *c, const double *dU, void *dv, int prec);
 /* zero the Dirichlet rows of CSR values (rows only) */
 int igab_launch_zero_csr_rows(igab_ctx *c, void *dv, int prec);

@@ -871,8 +871,8 @@ int launch_tan_volume_x(igab_ctx *c, const igab_geom &g, const double *dU, T *dv
 {
     if (c->phys == IGAB_PHYS_GETIME)
         return igab_launch_tan_getime(c, dU, dv, sizeof(T) == 8 ? IGAB_PREC_FP64 : IGAB_PREC_FP32);
-    if (sizeof(T) == 8 && c->tan_kernel == 1) return igab_launch_tan_dmma(c, dU, (double *)dv, tx0, tx1);
-    if (sizeof(T) == 4 && c->tan32_kernel == 1) return igab_launch_tan_tc32(c, dU, (float *)dv, tx0, tx1);
+    if ((sizeof(T) == 8 ? c->tan_kernel : c->tan32_kernel) == 1)
+        return igab_launch_tan_sf(c, dU, dv, sizeof(T) == 8 ? IGAB_PREC_FP64 : IGAB_PREC_FP32, tx0, tx1);
     return launch_tan_volume<T, 2>(c, g, dU, dv);
 }
 

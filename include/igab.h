@@ -128,9 +128,10 @@ int igab_check_finite(igab_ctx *ctx, const void *dev, long n, int prec, int *all
 
 /* ---- tuning: elements per tile edge of the 8-colour schedule (2 or 4), 0 = auto */
 int igab_set_tile(igab_ctx *ctx, int residual_tile, int tangent_tile);
-/* kernel choices: IGAB_OPT_TANGENT_FP64_KERNEL 1 = FP64 tensor path (mma f64), 0 = FP64 FMA pipe;
- * IGAB_OPT_TANGENT_FP32_KERNEL 1 = tcgen05 tensor cores (TF32 hi/lo split, FP32 accumulation in
- * tensor memory), 0 = FP32 FMA pipe.  IGAB_OPT_COLOUR_ORDER: the order in which the 8 colours
+/* kernel choices: IGAB_OPT_TANGENT_FP64_KERNEL 1 = sum factorisation on the FP64 tensor path (mma
+ * f64), 0 = direct form on the FP64 FMA pipe; IGAB_OPT_TANGENT_FP32_KERNEL 1 = the same sum
+ * factorisation with FP32 values (64-bit element matrices, rounded when they are added), 0 = direct
+ * form on the FP32 FMA pipe.  IGAB_OPT_COLOUR_ORDER: the order in which the 8 colours
  * of the element schedule are swept (colour = 4 x-parity + 2 y-parity + z-parity):
  * IGAB_COLOURS_NATURAL 0..7, IGAB_COLOURS_MIRRORED 3,2,1,0,7,6,5,4, IGAB_COLOURS_GRAY
  * 0,1,3,2,6,7,5,4.  Each order fixes the order in which every CSR entry receives its
@@ -157,15 +158,13 @@ int igab_fma_peak(int device, int prec, double *tflops);
 /* FP64 tensor-pipe throughput probe (TFLOP/s): back-to-back mma.sync m8n8k4 f64 on
  * independent accumulators, 32 warps per SM (the pipe of the FP64 tangent's products) */
 int igab_dmma_peak(int device, double *tflops);
-/* Check of the tcgen05 operand layout and descriptors used by the FP32 tensor-core tangent
- * (no reference counterpart): one CTA computes A B^T for fixed small-integer A (128 x 32) and
+/* Check of a tcgen05 operand layout and its descriptors (no reference counterpart): one CTA computes A B^T for fixed small-integer A (128 x 32) and
  * B (96 x 32) with the M 128 / N 96 and M 128 / N 32 instruction shapes; out (128 x 160 floats,
  * row-major) receives accumulator columns 0-95 (A B^T), 96-127 (A B[0:32]^T) and 128-159
  * (A B[0:32]^T over K 0-15 minus it over K 16-31, the negate-A form). */
 int igab_tc_selftest(int device, float *out);
 /* TF32 tensor-core throughput probe (TFLOP/s, dense): one CTA per SM issuing back-to-back
- * tcgen05.mma kind::tf32 M 128 x N n_cols x K 8 (n_cols 32, 96 = the FP32 tangent's
- * shapes, or 256 = full width); no reference counterpart. */
+ * tcgen05.mma kind::tf32 M 128 x N n_cols x K 8 (n_cols 32, 96 or 256 = full width); no reference counterpart. */
 int igab_tc_peak(int device, int n_cols, double *tflops);
 
 /* ---- CUDA graphs: capture one assembly at fixed device pointers, replay it.
@@ -198,7 +197,7 @@ int igab_adjoint_backward(igab_ctx *ctx, const double *U_dev, const void *vals_d
  * mesh and state (U_dev; NULL = zero state) with CUDA events on the context stream,
  * reps timed runs after one warm-up, and leaves the fastest applied.  what: bit 0
  * residual (elements per block: tile edge 2 or 4), bit 1 FP64 tangent (tensor path or FMA
- * pipe), bit 2 FP32 tangent (tcgen05 or FMA pipe), bit 3 colour order (the three orders of
+ * pipe), bit 2 FP32 tangent (the same two), bit 3 colour order (the three orders of
  * IGAB_OPT_COLOUR_ORDER, timed on the sum of the kernels bits 0-2 select, all three when
  * none).  Times of the chosen candidates in ms. */
 typedef struct {
