@@ -834,7 +834,7 @@ extern "C" int igab_history_jacobian_device(igab_ctx *ctx, const double *U_dev, 
     ctx->last_launches = 0;
     const size_t es = prec == IGAB_PREC_FP64 ? sizeof(double) : sizeof(float);
     IGAB_CUDA_TRY(cudaMemsetAsync(vals_dev, 0, (size_t)ctx->nnz * es, ctx->stream));
-    int rc = igab_launch_tan_getime_level(ctx, U_dev, vals_dev, prec, level);
+    int rc = igab_launch_tan_getime_level(ctx, U_dev, vals_dev, prec, level, 0, (ctx->ne[0] + 1) / 2);
     if (!rc) rc = igab_launch_zero_csr_rows(ctx, vals_dev, prec);
     return rc;
 }

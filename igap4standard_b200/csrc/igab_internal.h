@@ -36,7 +36,7 @@ struct igab_geom {
     const double *escale;
     /* phys/getime tangent-type assembly: weights w_j of the Hessian Taylor coefficients H_j
      * (j = 0..3) and the coefficient of the value-component mass term; the tangent d r/d u
-     * is w = (1/4, 1/6, 1/8, 0), mass rho/dt^2 + c/(2 dt) (igab_getime.cu) */
+     * is w = (1/4, 1/6, 1/8, 0), mass rho/dt^2 + c/(2 dt) (igab_tangent_sf.cu) */
     double tw[4];
     double tmass;
 };
@@ -236,11 +236,10 @@ int igab_launch_res_dirichlet_rows(long nd, const int *drow, const double *dg, c
 /* CTAs per SM the persistent kernels can hold */
 int igab_batch_occupancy_res(int *per_sm);
 int igab_batch_occupancy_tan(int prec, int *per_sm);
-int igab_launch_tan_getime(igab_ctx *c, const double *dU, void *dv, int prec);
 /* zero the Dirichlet rows of CSR values (rows only) */
 int igab_launch_zero_csr_rows(igab_ctx *c, void *dv, int prec);
-/* the same kernel with explicit weights (history Jacobians); level 0 = tangent */
-int igab_launch_tan_getime_level(igab_ctx *c, const double *dU, void *dv, int prec, int level);
+/* the transient tangent (level 0) or history Jacobian (level 1, 2), x tiles [tx0, tx1) */
+int igab_launch_tan_getime_level(igab_ctx *c, const double *dU, void *dv, int prec, int level, int tx0, int tx1);
 int igab_launch_exp_scale(igab_ctx *c, const double *dg);
 int igab_launch_adjoint_dRdg(igab_ctx *c, const double *dU, const double *dlam, double *dgrad);
 int igab_launch_tangent_transpose(igab_ctx *c, const void *dvals, int prec, const double *dx, double *dy);

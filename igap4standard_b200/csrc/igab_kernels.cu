@@ -869,9 +869,7 @@ int launch_tan_volume(igab_ctx *c, const igab_geom &g, const double *dU, T *dv)
 template <typename T>
 int launch_tan_volume_x(igab_ctx *c, const igab_geom &g, const double *dU, T *dv, int tx0, int tx1)
 {
-    if (c->phys == IGAB_PHYS_GETIME)
-        return igab_launch_tan_getime(c, dU, dv, sizeof(T) == 8 ? IGAB_PREC_FP64 : IGAB_PREC_FP32);
-    if ((sizeof(T) == 8 ? c->tan_kernel : c->tan32_kernel) == 1)
+    if (c->phys == IGAB_PHYS_GETIME || (sizeof(T) == 8 ? c->tan_kernel : c->tan32_kernel) == 1)
         return igab_launch_tan_sf(c, dU, dv, sizeof(T) == 8 ? IGAB_PREC_FP64 : IGAB_PREC_FP32, tx0, tx1);
     return launch_tan_volume<T, 2>(c, g, dU, dv);
 }
@@ -934,7 +932,7 @@ int launch_tangent_slabs_t(igab_ctx *c, const double *dU, T *dv, long *row_end, 
     igab_geom g = c->geom();
     const int ntx = (c->ne[0] + 1) / 2;
     int b[IGAB_MAX_SLABS];
-    const bool ranged = c->phys != IGAB_PHYS_GETIME && (sizeof(T) == 8 ? c->tan_kernel == 1 : c->tan32_kernel == 1);
+    const bool ranged = c->phys == IGAB_PHYS_GETIME || (sizeof(T) == 8 ? c->tan_kernel == 1 : c->tan32_kernel == 1);
     const int nb = ranged ? slab_bounds(ntx, b) : 0;
     for (int i = 0; i <= nb; i++)
         if (!c->slab_ev[i]) IGAB_CUDA_TRY(cudaEventCreateWithFlags(&c->slab_ev[i], cudaEventDisableTiming));

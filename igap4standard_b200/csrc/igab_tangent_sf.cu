@@ -28,10 +28,19 @@
  * beside the first step of the next, and the read-out of one component row and the next element's
  * field beside later pairs.
  *
- * Measured at 64^3 (tangent alone): 22.3 ms, FP64 and FP32 values, against 96.6 ms for the rank-12 form
- * on the same pipe and 40.4 ms for its TF32 tcgen05 form; the FP32 values' error against 64 bits falls
- * from 1.3e-6 to 8e-8.  Bound by shared memory (17,300 wavefronts per element, 60-70% of the rate);
- * the products take 7,500 cycles of the pipe.
+ * phys/getime uses the same kernel (NR = 2): its Hessian is a weighted sum over the Taylor orders of the segment
+ * from t_n-1/2 to t_n+1/2, which is the static form summed over two fields (sf_coef), plus the inertia term on
+ * the value components; the additional work is in the point matrices only.  FP64 throughout; FP32 values round
+ * at the store.
+ *
+ * Measured (tangent alone).  64^3: 20.5 ms, FP64 and FP32 values, against 96.6 ms for the rank-12 form on the
+ * same pipe and 40.4 ms for its TF32 tcgen05 form, whose values had 1.3e-6 error against 64 bits (8e-8 here).
+ * 32^3 transient: 6.1 ms against 33.7 ms for the rank-24 form.  Bound by instruction latency in the short
+ * barrier phases (IPC 0.36 per scheduler; tensor and FP64 pipe 47%).  Measured and left out: the second step fed
+ * from the first one's accumulators in registers, without T1 (23.0 ms: it moves the third step into the same
+ * warps' serial chain); totals by shuffles instead of a product with ones (+0.7 ms); one copy of each part
+ * of the code under run-time slots and phases (54 instead of 85 KB of code, +2.5 ms); padding of the element
+ * matrices against bank conflicts (no change).
  */
 #include <cuda_runtime.h>
 #include <type_traits>
@@ -100,27 +109,51 @@ __host__ __device__ constexpr int x_zwarp(bool diag, int X)
 }
 
 /* point data, [item][64 points], point = 4 (4 qx + qy) + qz; CN, S and TAU times the weight */
-enum { P_F = 0, P_G = 9, P_W = 27, P_CN = 28, P_S = 34, P_TAU = 40, P_N = 49 };
+template <int NR>
+struct pt_at {   /* NR = 1: phys/ge; 2: phys/getime, the two fields of the hat form */
+    static constexpr int NC = NR == 1 ? 1 : 3;   /* CN of the field pairs (0,0), (0,1), (1,1) */
+    static constexpr int F = 0, G = 9 * NR, W = 27 * NR, CN = W + 1, S = CN + 6 * NC, TAU = S + 6, N = TAU + 9;
+};
 
-struct sf_row { long rb; int rsx, rsy, len, pad; };
+/* material constants of D, and the hat form of the transient tangent: with the weights tw of the Hessian's
+ * Taylor coefficients, tw0 a a + 2 tw1 a b + tw2 b b = (r00 a + r01 b)^2 + (r11 b)^2, so that every term with a
+ * constant Phi'' is the static one summed over the two fields r00 m + r01 h and r11 h (igab_math.cuh: m, h);
+ * (al, be, ga) is the inverse map, mass the coefficient of the value components */
+struct sf_coef {
+    double aon, aoff, ash;
+    double r00, r01, r11, al, be, ga, mass;
+};
+__host__ __device__ inline sf_coef sf_coef_ge(const igab_geom &g)
+{
+    sf_coef C = {};
+    C.aon = g.coef.p4sq * (4.0 / 3.0);
+    C.aoff = g.coef.p4sq * (-2.0 / 3.0);
+    C.ash = g.coef.p3 * 0.5;
+    return C;
+}
 
+struct __align__(16) sf_row { long rb; int rsx, rsy; };
+
+template <int NR>
 struct sf_smem {
-    double pt[P_N * 64];
+    double pt[pt_at<NR>::N * 64];
     double T1[36 * 128];     /* [class pair][8 pairs (az,bz)][16 columns], 16-byte chunks swizzled */
-    double T1x[25 * 16];     /* z totals of the class pairs without z derivative */
+    double T1x[(24 + NR) * 16];   /* z totals of the class pairs without z derivative (and of the values) */
     double T2[9 * 288];      /* [kx,lx][9 (ay,by)][4 qx][8 (az,bz)], swizzled */
     double T2x[9 * 36];      /* z totals [kx,lx][9 (ay,by)][4 qx] */
     double K[4 * 729];       /* element matrices of component pairs, [9 (ax,bx)][9 (ay,by)][9 (az,bz)] */
     double tab[2][3][IGAB_TAB1D];
     double wh[2][3][IGAB_NQ];
     double esc[2];
-    sf_row row[27];
+    sf_row row[3][27];
 };
-/* the staging of the next element's field and the fifth element-matrix slot use T1 / T1x, which are free then */
+static_assert(sizeof(sf_smem<1>) + 1024 + 384 <= 233472 / 2, "two blocks per SM");
+/* the control values and the interpolation of the next element's field and the fifth element-matrix slot use
+ * T1x and T1, which are free then */
+#define SF_U(S, f) ((S).T1x + 82 * (f))
 #define SF_A(S) ((S).T1)
-#define SF_C(S) ((S).T1 + 972)
-#define SF_U(S) ((S).T1x)
-#define SF_KSLOT(S, s) ((s) < 4 ? (S).K + 729 * (s) : (S).T1 + 2048)
+#define SF_C(S) ((S).T1 + 648)
+#define SF_KSLOT(S, s) ((s) < 4 ? (S).K + 729 * (s) : (S).T1 + 2400)
 
 /* f(integral_constant 0), ..., f(integral_constant N - 1) */
 template <int I, int N, class F>
@@ -138,11 +171,6 @@ __device__ __forceinline__ void sf_dmma(double &c0, double &c1, double a, double
         : "+d"(c0), "+d"(c1)
         : "d"(a), "d"(b));
 }
-__device__ __forceinline__ double sum4(double v)
-{
-    v += shfl_xor(v, 1);
-    return v + shfl_xor(v, 2);
-}
 /* the pair index 3 a + b of row r of an m8 tile (all but 4 = (1, 1)) */
 __device__ __forceinline__ int pair_id(int r) { return r + (r >> 2); }
 
@@ -159,97 +187,129 @@ __device__ __forceinline__ void sf_weights(const double *tab, int lane, double w
 }
 
 /* one point's data of a component pair */
+template <int NR>
 struct sf_point {
-    double f[3], h[3], g[6], y[6];   /* F and second derivatives of k and l */
-    double won, woff, wsh;           /* w * 2 le^2 (2/3, -1/3), w * e345 / 2 */
-    double cn[6], s[6], tau[9];
+    double f[NR][3], h[NR][3], g[NR][6], y[NR][6];   /* F and second derivatives of k and l */
+    double won, woff, wsh;                           /* w * 2 le^2 (2/3, -1/3), w * e345 / 2 */
+    double cn[pt_at<NR>::NC][6], s[6], tau[9];
 };
 
 /* w D_mn of the point */
-template <bool DG, int m, int n>
-__device__ __forceinline__ double sf_d(const sf_point &P)
+template <int NR, bool DG, int m, int n>
+__device__ __forceinline__ double sf_d(const sf_point<NR> &P)
 {
+    double v = 0.0;
     if constexpr (m < 3 && n < 3) {
-        constexpr int I = m, J = n, M1 = (I + 1) % 3, M2 = (I + 2) % 3;
-        const double t = P.g[sym6(I, 0)] * P.y[sym6(J, 0)] + P.g[sym6(I, 1)] * P.y[sym6(J, 1)] +
-                         P.g[sym6(I, 2)] * P.y[sym6(J, 2)];
-        double v = (I == J ? P.won : P.woff) * t + P.cn[sym6(I, J)] * (P.f[I] * P.h[J]);
-        if constexpr (I != J) v += P.wsh * (P.f[J] * P.h[I]);
-        else v += P.wsh * (P.f[M1] * P.h[M1] + P.f[M2] * P.h[M2]);
-        if constexpr (DG) v += P.s[sym6(I, J)];
-        return v;
+        constexpr int I = m, J = n, M1 = (I + 1) % 3, M2 = (I + 2) % 3, IJ = sym6(I, J);
+        double t = 0.0, u = 0.0;
+#pragma unroll
+        for (int r = 0; r < NR; r++) {
+            t += P.g[r][sym6(I, 0)] * P.y[r][sym6(J, 0)] + P.g[r][sym6(I, 1)] * P.y[r][sym6(J, 1)] +
+                 P.g[r][sym6(I, 2)] * P.y[r][sym6(J, 2)];
+            if constexpr (I != J) u += P.f[r][J] * P.h[r][I];
+            else u += P.f[r][M1] * P.h[r][M1] + P.f[r][M2] * P.h[r][M2];
+        }
+        v = (I == J ? P.won : P.woff) * t + P.cn[0][IJ] * (P.f[0][I] * P.h[0][J]);
+        v += P.wsh * u;
+        if constexpr (NR == 2)
+            v += P.cn[1][IJ] * (P.f[0][I] * P.h[1][J] + P.f[1][I] * P.h[0][J]) + P.cn[2][IJ] * (P.f[1][I] * P.h[1][J]);
+        if constexpr (DG) v += P.s[IJ];
     } else if constexpr (m < 3) {
         constexpr int I = m, J = s_i(n - 3), K = s_k(n - 3);
-        double v = P.g[sym6(I, K)] * ((I == J ? P.won : P.woff) * P.h[J]);
-        if constexpr (J != K) v += P.g[sym6(I, J)] * ((I == K ? P.won : P.woff) * P.h[K]);
+#pragma unroll
+        for (int r = 0; r < NR; r++) {
+            v += P.g[r][sym6(I, K)] * ((I == J ? P.won : P.woff) * P.h[r][J]);
+            if constexpr (J != K) v += P.g[r][sym6(I, J)] * ((I == K ? P.won : P.woff) * P.h[r][K]);
+        }
         if constexpr (DG && I == J) v += P.tau[3 * I + K];
         else if constexpr (DG && I == K) v += P.tau[3 * I + J];
-        return v;
     } else if constexpr (n < 3) {
         constexpr int J = n, I = s_i(m - 3), K = s_k(m - 3);
-        double v = ((I == J ? P.won : P.woff) * P.f[I]) * P.y[sym6(J, K)];
-        if constexpr (I != K) v += ((K == J ? P.won : P.woff) * P.f[K]) * P.y[sym6(J, I)];
+#pragma unroll
+        for (int r = 0; r < NR; r++) {
+            v += ((I == J ? P.won : P.woff) * P.f[r][I]) * P.y[r][sym6(J, K)];
+            if constexpr (I != K) v += ((K == J ? P.won : P.woff) * P.f[r][K]) * P.y[r][sym6(J, I)];
+        }
         if constexpr (DG && J == I) v += P.tau[3 * J + K];
         else if constexpr (DG && J == K) v += P.tau[3 * J + I];
-        return v;
     } else {
         /* over the orderings (I, K) of m and (J, L) of n with K = L: A_IJ f_I h_J */
         constexpr int i0 = s_i(m - 3), k0 = s_k(m - 3), j0 = s_i(n - 3), l0 = s_k(n - 3);
-        double v = 0.0;
-        if constexpr (k0 == l0) v += P.f[i0] * ((i0 == j0 ? P.won : P.woff) * P.h[j0]);
-        if constexpr (i0 != k0 && i0 == l0) v += P.f[k0] * ((k0 == j0 ? P.won : P.woff) * P.h[j0]);
-        if constexpr (j0 != l0 && k0 == j0) v += P.f[i0] * ((i0 == l0 ? P.won : P.woff) * P.h[l0]);
-        if constexpr (i0 != k0 && j0 != l0 && i0 == j0) v += P.f[k0] * ((k0 == l0 ? P.won : P.woff) * P.h[l0]);
-        return v;
+#pragma unroll
+        for (int r = 0; r < NR; r++) {
+            if constexpr (k0 == l0) v += P.f[r][i0] * ((i0 == j0 ? P.won : P.woff) * P.h[r][j0]);
+            if constexpr (i0 != k0 && i0 == l0) v += P.f[r][k0] * ((k0 == j0 ? P.won : P.woff) * P.h[r][j0]);
+            if constexpr (j0 != l0 && k0 == j0) v += P.f[r][i0] * ((i0 == l0 ? P.won : P.woff) * P.h[r][l0]);
+            if constexpr (i0 != k0 && j0 != l0 && i0 == j0)
+                v += P.f[r][k0] * ((k0 == l0 ? P.won : P.woff) * P.h[r][l0]);
+        }
     }
+    return v;
 }
 
 /* first step: the class pairs of group G, for the 8 columns of half h */
-template <int G, bool DG>
-__device__ __forceinline__ void sf_s1(sf_smem &S, const double *tz, int lane, int h, int k, int l, double aon,
-                                      double aoff, double ash)
+template <int NR, int G, bool DG>
+__device__ __forceinline__ void sf_s1(sf_smem<NR> &S, const double *tz, int lane, int h, int k, int l, const sf_coef &C)
 {
     double w[9];
     sf_weights(tz, lane, w);
     const double *p = S.pt + h * 32 + lane;
-    sf_point P;
+    using A = pt_at<NR>;
+    sf_point<NR> P;
 #pragma unroll
-    for (int J = 0; J < 3; J++) {
-        P.f[J] = p[(P_F + 3 * k + J) * 64];
-        P.h[J] = DG ? P.f[J] : p[(P_F + 3 * l + J) * 64];
+    for (int r = 0; r < NR; r++) {
+#pragma unroll
+        for (int J = 0; J < 3; J++) {
+            P.f[r][J] = p[(A::F + 9 * r + 3 * k + J) * 64];
+            P.h[r][J] = DG ? P.f[r][J] : p[(A::F + 9 * r + 3 * l + J) * 64];
+        }
+#pragma unroll
+        for (int c = 0; c < 6; c++) {
+            P.g[r][c] = p[(A::G + 18 * r + 6 * k + c) * 64];
+            P.y[r][c] = DG ? P.g[r][c] : p[(A::G + 18 * r + 6 * l + c) * 64];
+        }
     }
 #pragma unroll
     for (int c = 0; c < 6; c++) {
-        P.g[c] = p[(P_G + 6 * k + c) * 64];
-        P.y[c] = DG ? P.g[c] : p[(P_G + 6 * l + c) * 64];
-        P.cn[c] = p[(P_CN + c) * 64];
-        P.s[c] = DG ? p[(P_S + c) * 64] : 0.0;
+#pragma unroll
+        for (int r = 0; r < A::NC; r++) P.cn[r][c] = p[(A::CN + 6 * r + c) * 64];
+        P.s[c] = DG ? p[(A::S + c) * 64] : 0.0;
     }
 #pragma unroll
-    for (int c = 0; c < 9; c++) P.tau[c] = DG ? p[(P_TAU + c) * 64] : 0.0;
-    const double wq = p[P_W * 64];
-    P.won = wq * aon;
-    P.woff = wq * aoff;
-    P.wsh = wq * ash;
-    const int r = lane >> 2;
+    for (int c = 0; c < 9; c++) P.tau[c] = DG ? p[(A::TAU + c) * 64] : 0.0;
+    const double wq = p[A::W * 64];
+    P.won = wq * C.aon;
+    P.woff = wq * C.aoff;
+    P.wsh = wq * C.ash;
+    const int r = lane >> 2, q = lane & 3;
     /* row r, chunk 4 h + lane % 4 of two columns; chunks are XORed so that these stores and the second
      * step's loads (4 rows x 4 qy) hit distinct banks */
-    double *t1 = S.T1 + r * 16 + 2 * ((4 * h + (lane & 3)) ^ (4 * (r & 1) + (r & 2)));
-    double *t1x = S.T1x + 8 * h + r;
+    double *t1 = S.T1 + r * 16 + 2 * ((4 * h + q) ^ (4 * (r & 1) + (r & 2)));
+    double *t1x = S.T1x + 8 * h + 2 * q;
     static_for<0, 36>([&](auto cd_) {
         constexpr int cd = decltype(cd_)::value, c = cd / 6, d = cd % 6;
         if constexpr (cls_nonzero(c, d) && !(DG && c > d) && cls_group(DG, c, d) == G) {
             double c0 = 0.0, c1 = 0.0;
+            if constexpr (NR == 2 && DG && cd == 0) {
+                /* inertia / damping: the value components, T1x row 25 */
+                const double v = 0.5 * C.mass * wq;
+                double t0 = 0.0, t1v = 0.0;
+                sf_dmma(c0, c1, w[0], v);
+                sf_dmma(t0, t1v, 1.0, v);
+                if (r == 0) *reinterpret_cast<double2 *>(t1x + 25 * 16) = make_double2(t0, t1v);
+            }
             static_for<0, 9>([&](auto kk_) {
-                constexpr int kk = decltype(kk_)::value, kz = kk / 3, lz = kk % 3, m = sf_comp(c, kz), n = sf_comp(d, lz);
+                constexpr int kk = decltype(kk_)::value, m = sf_comp(c, kk / 3), n = sf_comp(d, kk % 3);
                 if constexpr (m >= 0 && n >= 0) {
                     if constexpr (mn_nonzero(m, n) && !(DG && !mn_upper(m, n))) {
-                        double v = sf_d<DG, m, n>(P);
+                        double v = sf_d<NR, DG, m, n>(P);
                         if constexpr (DG && m == n) v *= 0.5;
                         sf_dmma(c0, c1, w[kk], v);
                         if constexpr (kk == 0) {
-                            const double t = sum4(v);
-                            if ((lane & 3) == 0) t1x[((c - 1) * 5 + d - 1) * 16] = t;
+                            double t0 = 0.0, t1v = 0.0;
+                            sf_dmma(t0, t1v, 1.0, v);
+                            if (r == 0)
+                                *reinterpret_cast<double2 *>(t1x + ((c - 1) * 5 + d - 1) * 16) = make_double2(t0, t1v);
                         }
                     }
                 }
@@ -259,9 +319,10 @@ __device__ __forceinline__ void sf_s1(sf_smem &S, const double *tz, int lane, in
     });
 }
 
-/* second step: the (kx, lx) of the half, for one qx */
-template <int HALF, bool DG>
-__device__ __forceinline__ void sf_s2(sf_smem &S, const double *ty, int lane, int qx)
+/* second step: the (kx, lx) of the half, for one qx; the z totals of a (kx, lx) by one warp of the half, with
+ * the four qx as columns */
+template <int NR, int HALF, bool DG>
+__device__ __forceinline__ void sf_s2(sf_smem<NR> &S, const double *ty, int lane, int qx)
 {
     double w[9];
     sf_weights(ty, lane, w);
@@ -270,8 +331,9 @@ __device__ __forceinline__ void sf_s2(sf_smem &S, const double *ty, int lane, in
     const int id = pair_id(n);
     /* T2 row (ay,by), 8 doubles per qx: qx flips with the row's parity and the (az,bz) halves with qx / 2,
      * so that 2-row stores and 4-qx loads hit distinct banks */
-    double *t2 = S.T2 + id * 32 + ((qx ^ (id & 1)) << 3) + ((2 * q) ^ (4 * (qx >> 1)));
-    double *t2y = S.T2 + 4 * 32 + (qx << 3) + (n ^ (4 * (qx >> 1)));
+    const int sw = (2 * q) ^ (4 * (qx >> 1));
+    double *t2 = S.T2 + id * 32 + ((qx ^ (id & 1)) << 3) + sw;
+    double *t2y = S.T2 + 4 * 32 + (qx << 3) + sw;
     static_for<0, 9>([&](auto X_) {
         constexpr int X = decltype(X_)::value, kx = X / 3, lx = X % 3;
         if constexpr (!(DG && kx > lx) && x_half(DG, X) == HALF) {
@@ -282,25 +344,28 @@ __device__ __forceinline__ void sf_s2(sf_smem &S, const double *ty, int lane, in
                     const double b = t1[cd * 128];
                     sf_dmma(c0, c1, w[kl], b);
                     if constexpr (kl == 0) {
-                        const double t = sum4(b);
-                        if (q == 0) t2y[X * 288] = t;
+                        double t0 = 0.0, t1v = 0.0;
+                        sf_dmma(t0, t1v, 1.0, b);
+                        if (n == 0) *reinterpret_cast<double2 *>(t2y + X * 288) = make_double2(t0, t1v);
                     }
                 }
             });
             *reinterpret_cast<double2 *>(t2 + X * 288) = make_double2(c0, c1);
             if (qx == x_zwarp(DG, X)) {
-                /* z totals, all four qx as columns */
                 const double *t1x = S.T1x + (n & 3) * 4 + q;
                 c0 = c1 = 0.0;
                 static_for<0, 36>([&](auto cd_) {
                     constexpr int cd = decltype(cd_)::value, c = cd / 6, d = cd % 6, kl = 3 * cls_ky(c) + cls_ky(d);
-                    if constexpr (c > 0 && d > 0 && cls_kx(c) == kx && cls_kx(d) == lx && cls_nonzero(c, d) &&
-                                  !(DG && c > d)) {
-                        const double b = n < 4 ? t1x[((c - 1) * 5 + d - 1) * 16] : 0.0;
+                    constexpr bool mass = NR == 2 && DG && cd == 0;
+                    if constexpr (((c > 0 && d > 0) || mass) && cls_kx(c) == kx && cls_kx(d) == lx &&
+                                  cls_nonzero(c, d) && !(DG && c > d)) {
+                        const double b = n < 4 ? t1x[(mass ? 25 : (c - 1) * 5 + d - 1) * 16] : 0.0;
                         sf_dmma(c0, c1, w[kl], b);
                         if constexpr (kl == 0) {
-                            const double t = sum4(b);
-                            if (q == 0 && n < 4) S.T2x[X * 36 + 16 + n] = t;
+                            double t0 = 0.0, t1v = 0.0;
+                            sf_dmma(t0, t1v, 1.0, b);
+                            if (lane < 2)
+                                *reinterpret_cast<double2 *>(S.T2x + X * 36 + 16 + 2 * q) = make_double2(t0, t1v);
                         }
                     }
                 });
@@ -310,64 +375,91 @@ __device__ __forceinline__ void sf_s2(sf_smem &S, const double *ty, int lane, in
     });
 }
 
-/* third step into an element-matrix slot: one tile of eight (az,bz) columns per (ay,by), then the z totals */
+/* third step: the tile of eight (az,bz) columns of (ay,by) t; all loads first, then two product chains */
 template <bool DG>
-__device__ __forceinline__ void sf_s3(sf_smem &S, const double *tx, double *K, int warp, int lane)
+__device__ __forceinline__ void sf_s3(const double *T2, const double w[9], double *K, int t, int lane)
+{
+    const int n = lane >> 2, q = lane & 3;
+    const double *t2 = T2 + t * 32 + ((q ^ (t & 1)) << 3) + (n ^ (4 * (q >> 1)));
+    double b[9], c0 = 0.0, c1 = 0.0, d0 = 0.0, d1 = 0.0, x0 = 0.0, x1 = 0.0;
+#pragma unroll
+    for (int X = 0; X < 9; X++)
+        if (!(DG && X / 3 > X % 3)) b[X] = t2[X * 288];
+#pragma unroll
+    for (int X = 0; X < 9; X++) {
+        if (DG && X / 3 > X % 3) continue;
+        if (X & 1) sf_dmma(d0, d1, w[X], b[X]);
+        else sf_dmma(c0, c1, w[X], b[X]);
+        if (X == 0) sf_dmma(x0, x1, 1.0, b[X]);
+    }
+    const int z0 = pair_id(2 * q), z1 = pair_id(2 * q + 1);
+    double *o = K + pair_id(n) * 81 + t * 9;
+    o[z0] = c0 + d0;
+    o[z1] = c1 + d1;
+    if (n == 0) {
+        K[4 * 81 + t * 9 + z0] = x0;
+        K[4 * 81 + t * 9 + z1] = x1;
+    }
+}
+
+/* third step of the z totals: job 9 the eight (ay,by), job 10 the total in y and z (only where both
+ * derivatives are in x, or of the values) */
+template <int NR, bool DG>
+__device__ __forceinline__ void sf_s3z(const double *T2x, const double w[9], double *K, int job, int lane)
+{
+    const int n = lane >> 2, q = lane & 3, xr = pair_id(n) * 81;
+    double c0 = 0.0, c1 = 0.0;
+    if (job == 9) {
+        const double *t2 = T2x + pair_id(n) * 4 + q;
+        double t0 = 0.0, t1 = 0.0;
+#pragma unroll
+        for (int X = 0; X < 9; X++) {
+            if (DG && X / 3 > X % 3) continue;
+            const double b = t2[X * 36];
+            sf_dmma(c0, c1, w[X], b);
+            if (X == 0) sf_dmma(t0, t1, 1.0, b);
+        }
+        K[xr + pair_id(2 * q) * 9 + 4] = c0;
+        K[xr + pair_id(2 * q + 1) * 9 + 4] = c1;
+        if (n == 0) {
+            K[4 * 81 + pair_id(2 * q) * 9 + 4] = t0;
+            K[4 * 81 + pair_id(2 * q + 1) * 9 + 4] = t1;
+        }
+    } else {
+        double t0 = 0.0, t1 = 0.0;
+#pragma unroll
+        for (int X = 0; X < 9; X++) {
+            const bool mass = NR == 2 && DG && X == 0;
+            if (!mass && (X / 3 == 0 || X % 3 == 0 || (DG && X / 3 > X % 3))) continue;
+            const double b = n == 0 ? T2x[X * 36 + 16 + q] : 0.0;
+            sf_dmma(c0, c1, w[X], b);
+            if (mass) sf_dmma(t0, t1, 1.0, b);
+        }
+        if (q == 0) K[xr + 4 * 9 + 4] = c0;
+        if (lane == 0) K[4 * 81 + 4 * 9 + 4] = t0;
+    }
+}
+
+/* third step of a pair into an element-matrix slot: tiles 0-8, then the z totals, over the warps */
+template <int NR, bool DG>
+__device__ __forceinline__ void sf_s3_all(sf_smem<NR> &S, const double *tx, double *K, int warp, int lane)
 {
     double w[9];
     sf_weights(tx, lane, w);
-    const int n = lane >> 2, q = lane & 3;
-    const int xr = pair_id(n) * 81;
+#pragma unroll 1
     for (int t = warp; t < 11; t += 8) {
-        double c0 = 0.0, c1 = 0.0;
-        if (t < 9) {
-            const double *t2 = S.T2 + t * 32 + ((q ^ (t & 1)) << 3) + (n ^ (4 * (q >> 1)));
-#pragma unroll
-            for (int X = 0; X < 9; X++) {
-                if (DG && X / 3 > X % 3) continue;
-                const double b = t2[X * 288];
-                sf_dmma(c0, c1, w[X], b);
-                if (X == 0) {
-                    const double s = sum4(b);
-                    if (q == 0) K[4 * 81 + t * 9 + pair_id(n)] = s;
-                }
-            }
-            K[xr + t * 9 + pair_id(2 * q)] = c0;
-            K[xr + t * 9 + pair_id(2 * q + 1)] = c1;
-        } else if (t == 9) {
-            const double *t2 = S.T2x + pair_id(n) * 4 + q;
-#pragma unroll
-            for (int X = 0; X < 9; X++) {
-                if (DG && X / 3 > X % 3) continue;
-                const double b = t2[X * 36];
-                sf_dmma(c0, c1, w[X], b);
-                if (X == 0) {
-                    const double s = sum4(b);
-                    if (q == 0) K[4 * 81 + pair_id(n) * 9 + 4] = s;
-                }
-            }
-            K[xr + pair_id(2 * q) * 9 + 4] = c0;
-            K[xr + pair_id(2 * q + 1) * 9 + 4] = c1;
-        } else {
-            /* totals in y and z: only where both derivatives are in x */
-#pragma unroll
-            for (int X = 0; X < 9; X++) {
-                if (X / 3 == 0 || X % 3 == 0 || (DG && X / 3 > X % 3)) continue;
-                const double b = n == 0 ? S.T2x[X * 36 + 16 + q] : 0.0;
-                sf_dmma(c0, c1, w[X], b);
-            }
-            if (q == 0) K[xr + 4 * 9 + 4] = c0;
-            if (lane == 0) K[4 * 81 + 4 * 9 + 4] = 0.0;
-        }
+        if (t < 9) sf_s3<DG>(S.T2, w, K, t, lane);
+        else sf_s3z<NR, DG>(S.T2x, w, K, t, lane);
     }
 }
 
 /* totals -> entries (1, 1) in z, then y, of slots s0, s1, s2 (the first ns): a warp per three (ax,bx) */
-__device__ __forceinline__ void sf_fix_zy(sf_smem &S, int s0, int s1, int s2, int ns, int warp, int lane)
+template <int NR>
+__device__ __forceinline__ void sf_fix_zy(sf_smem<NR> &S, int s0, int s1, int s2, int ns, int warp, int lane)
 {
     for (int u = warp; u < 3 * ns; u += 8) {
-        const int sl = u / 3, j = u % 3;
-        double *K = SF_KSLOT(S, sl == 0 ? s0 : (sl == 1 ? s1 : s2)) + (3 * j + lane / 9) * 81;
+        const int sl = u / 3;
+        double *K = SF_KSLOT(S, sl == 0 ? s0 : (sl == 1 ? s1 : s2)) + (3 * (u - 3 * sl) + lane / 9) * 81;
         const int e = lane % 9;
         if (lane < 27) {
             double *z = K + e * 9;
@@ -381,20 +473,21 @@ __device__ __forceinline__ void sf_fix_zy(sf_smem &S, int s0, int s1, int s2, in
     }
 }
 /* and in x */
-__device__ __forceinline__ void sf_fix_x(sf_smem &S, int s0, int s1, int s2, int ns, int tid)
+template <int NR>
+__device__ __forceinline__ void sf_fix_x(sf_smem<NR> &S, int s0, int s1, int s2, int ns, int tid)
 {
     if (tid < 81 * ns) {
         const int sl = tid / 81;
-        double *z = SF_KSLOT(S, sl == 0 ? s0 : (sl == 1 ? s1 : s2)) + tid % 81;
+        double *z = SF_KSLOT(S, sl == 0 ? s0 : (sl == 1 ? s1 : s2)) + (tid - 81 * sl);
         z[324] -= ((z[0] + z[81]) + (z[162] + z[243])) + ((z[405] + z[486]) + (z[567] + z[648]));
     }
 }
 
-/* Add rows (a, k), a = 0..26, into the CSR values: sl[l] is the slot of pair (min(k,l), max(k,l)).
- * A thread owns one column c2 = 3 b + l and walks the 9 rows of one ax, so consecutive lanes add to runs
- * of 9 consecutive values and the index arithmetic of a row is three multiply-adds. */
-template <typename T>
-__device__ __forceinline__ void sf_scatter(sf_smem &S, T *__restrict__ vals, int k, int s0, int s1, int s2, int tid)
+/* Add rows (a, k), a = 0..26, into the CSR values; slot s_l holds pair (min(k,l), max(k,l)).  A thread owns one column c2 = 3 b + l and walks the 9
+ * rows of one ax, so consecutive lanes add to runs of 9 consecutive values and the index arithmetic of a row
+ * is two multiply-adds. */
+template <typename T, int NR>
+__device__ __forceinline__ void sf_scatter(sf_smem<NR> &S, T *__restrict__ vals, int k, int s0, int s1, int s2, int tid)
 {
     if (tid >= 243) return;
     const int j = tid / 81, c = tid - 81 * j, l = c % 3, b = c / 3;
@@ -402,153 +495,274 @@ __device__ __forceinline__ void sf_scatter(sf_smem &S, T *__restrict__ vals, int
     const double *Kl = SF_KSLOT(S, l == 0 ? s0 : (l == 1 ? s1 : s2));
     const double *Kn = Kl + (3 * j + bx) * 81 + by * 9 + bz;       /* (a, b), + 27 ay + 3 az */
     const double *Kt = Kl + (3 * bx + j) * 81 + by * 27 + bz * 3;  /* (b, a), + 9 ay + az */
+    const bool up = l >= k, dg = l == k;
+    const double *Ka = up ? Kn : Kt;
+    const int sy = up ? 27 : 9, sz = up ? 3 : 1;
+    double x[9];
+#pragma unroll
+    for (int a = 0; a < 9; a++) x[a] = Ka[(a / 3) * sy + (a % 3) * sz];
+    if (dg)
+#pragma unroll
+        for (int a = 0; a < 9; a++) x[a] += Kt[9 * (a / 3) + a % 3];
     T *v = vals + c % 9;
 #pragma unroll
-    for (int ay = 0; ay < 3; ay++)
-#pragma unroll
-        for (int az = 0; az < 3; az++) {
-            const sf_row &R = S.row[9 * j + 3 * ay + az];
-            double x = l >= k ? Kn[27 * ay + 3 * az] : Kt[9 * ay + az];
-            if (l == k) x += Kt[9 * ay + az];
-            atomicAdd(v + R.rb + k * R.len + bx * R.rsx + by * R.rsy, T(x));
-        }
+    for (int a = 0; a < 9; a++) {
+        const sf_row R = S.row[k][9 * j + a];
+        atomicAdd(v + R.rb + (bx * R.rsx + by * R.rsy), T(x[a]));
+    }
 }
 
 /* ---- the field of an element: loads, three interpolation steps, point data */
 struct sf_elem { int ex, ey, ez; };
 
-/* one value per thread: 81 of U, 108 of the 1-D tables, 12 weights, the element scale */
-__device__ __forceinline__ double sf_prefetch(const igab_geom &g, const double *__restrict__ U, const sf_elem &E,
-                                              int tid)
+__device__ __forceinline__ void sf_copy8(double *dst, const double *src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void sf_copy_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+/* asynchronous loads of an element: U (and the two history levels), the 1-D tables, weights, the scale */
+template <int NR>
+__device__ __forceinline__ void sf_load(sf_smem<NR> &S, const igab_geom &g, const double *__restrict__ U, const sf_elem &E,
+                                        int buf, int tid)
 {
     if (tid < 81) {
         const int i = tid % 3, a = tid / 3;
-        return U[3 * cp_index(g, E.ex + a / 9, E.ey + (a / 3) % 3, E.ez + a % 3) + i];
-    }
-    if (tid < 189) {
+        const long o = 3 * cp_index(g, E.ex + a / 9, E.ey + (a / 3) % 3, E.ez + a % 3) + i;
+        sf_copy8(SF_U(S, 0) + tid, U + o);
+        if constexpr (NR == 2) {
+            sf_copy8(SF_U(S, 1) + tid, g.hist1 + o);
+            sf_copy8(SF_U(S, 2) + tid, g.hist0 + o);
+        }
+    } else if (tid < 189) {
         const int d = (tid - 81) / 36, o = (tid - 81) % 36, e = d == 0 ? E.ex : (d == 1 ? E.ey : E.ez);
-        return g.tab[d][(long)e * IGAB_TAB1D + o];
-    }
-    if (tid < 201) {
+        sf_copy8(&S.tab[buf][d][o], g.tab[d] + (long)e * IGAB_TAB1D + o);
+    } else if (tid < 201) {
         const int d = (tid - 189) >> 2, o = (tid - 189) & 3, e = d == 0 ? E.ex : (d == 1 ? E.ey : E.ez);
-        return g.wh[d][(long)e * IGAB_NQ + o];
+        sf_copy8(&S.wh[buf][d][o], g.wh[d] + (long)e * IGAB_NQ + o);
+    } else if (tid == 201) {
+        if (g.escale) sf_copy8(&S.esc[buf], g.escale + ((long)E.ex * g.ne[1] + E.ey) * g.ne[2] + E.ez);
+        else S.esc[buf] = 1.0;
     }
-    return tid == 201 ? elem_scale(g, E.ex, E.ey, E.ez) : 0.0;
 }
-__device__ __forceinline__ void sf_stage(sf_smem &S, double v, int buf, int tid)
+/* field r of control value o: U, or the middle (u0 + u1) / 2 and the half step (u - u0) / 2 */
+template <int NR>
+__device__ __forceinline__ double sf_value(const sf_smem<NR> &S, int r, int o)
 {
-    if (tid < 81) SF_U(S)[tid] = v;
-    else if (tid < 189) (&S.tab[buf][0][0])[tid - 81] = v;
-    else if (tid < 201) (&S.wh[buf][0][0])[tid - 189] = v;
-    else if (tid == 201) S.esc[buf] = v;
+    if (NR == 1) return SF_U(S, 0)[o];
+    return 0.5 * (r == 0 ? SF_U(S, 2)[o] + SF_U(S, 1)[o] : SF_U(S, 0)[o] - SF_U(S, 2)[o]);
 }
-__device__ __forceinline__ void sf_interp_z(sf_smem &S, int buf, int tid)
+template <int NR>
+__device__ __forceinline__ void sf_interp_z(sf_smem<NR> &S, int buf, int tid)
 {
     const double *Bz = S.tab[buf][2];
-    for (int o = tid; o < 972; o += SF_THR) {
-        const int i = o % 3, kz = (o / 3) % 3, a = (o / 9) % 9, q = o / 81;
-        const double *u0 = SF_U(S) + a * 9 + i;
-        SF_A(S)[o] = Bz[q * 9 + kz] * u0[0] + Bz[q * 9 + 3 + kz] * u0[3] + Bz[q * 9 + 6 + kz] * u0[6];
+    for (int o = tid; o < 324 * NR; o += SF_THR) {
+        const int f = o / 324, e = o - 324 * f, i = e % 3, kz = (e / 3) % 3, a = ((e / 9) % 9) * 9 + i, q = e / 81;
+        SF_A(S)[o] = Bz[q * 9 + kz] * sf_value<NR>(S, f, a) + Bz[q * 9 + 3 + kz] * sf_value<NR>(S, f, a + 3) +
+                     Bz[q * 9 + 6 + kz] * sf_value<NR>(S, f, a + 6);
     }
 }
-__device__ __forceinline__ void sf_interp_y(sf_smem &S, int buf, int tid)
+template <int NR>
+__device__ __forceinline__ void sf_interp_y(sf_smem<NR> &S, int buf, int tid)
 {
     const double *By = S.tab[buf][1];
-    for (int o = tid; o < 864; o += SF_THR) {
-        const int i = o % 3, kk = (o / 3) % 6, ax = (o / 18) % 3, qq = o / 54;
+    for (int o = tid; o < 864 * NR; o += SF_THR) {
+        const int f = o / 864, e = o - 864 * f;
+        const int i = e % 3, kk = (e / 3) % 6, ax = (e / 18) % 3, qq = e / 54;
         const int qy = qq & 3, qz = qq >> 2, ky = kk_ky(kk), kz = kk_kz(kk);
-        const double *a0 = SF_A(S) + ((qz * 3 + ax) * 3) * 9 + kz * 3 + i;
+        const double *a0 = SF_A(S) + 324 * f + ((qz * 3 + ax) * 3) * 9 + kz * 3 + i;
         SF_C(S)[o] = By[qy * 9 + ky] * a0[0] + By[qy * 9 + 3 + ky] * a0[9] + By[qy * 9 + 6 + ky] * a0[18];
     }
 }
-/* F and G of component tid / 64 at point tid % 64 */
-__device__ __forceinline__ void sf_interp_x(sf_smem &S, const igab_geom &g, int buf, int tid)
+/* F and G of component tid / 64 at point tid % 64; for NR = 2 of the hat fields r00 m + r01 h, r11 h */
+template <int NR>
+__device__ __forceinline__ void sf_interp_x(sf_smem<NR> &S, const igab_geom &g, const sf_coef &R, int buf, int tid)
 {
     if (tid >= 192) return;
+    using A = pt_at<NR>;
     const int i = tid >> 6, p = tid & 63, qz = p & 3, qy = (p >> 2) & 3, qx = p >> 4;
-    const double *C = SF_C(S) + (qy + 4 * qz) * 54 + i;
     const double *Bx = S.tab[buf][0] + qx * 9;
-    double b[3][3];
+    double b[3][3], u[NR][9];
 #pragma unroll
     for (int ax = 0; ax < 3; ax++)
 #pragma unroll
         for (int k = 0; k < 3; k++) b[ax][k] = Bx[ax * 3 + k];
 #pragma unroll
-    for (int a = 1; a < 10; a++) {
-        double s = 0.0;
+    for (int f = 0; f < NR; f++) {
+        const double *C = SF_C(S) + 864 * f + (qy + 4 * qz) * 54 + i;
+        double c[3][6];
 #pragma unroll
-        for (int ax = 0; ax < 3; ax++) s += b[ax][a_kx(a)] * C[(ax * 6 + a_kk(a)) * 3];
-        if (a < 4) {
-            if (g.periodic) s += g.pp[3 * i + a - 1];
-            if (i == a - 1) s += 1.0;
-            S.pt[(P_F + 3 * i + a - 1) * 64 + p] = s;
-        } else
-            S.pt[(P_G + 6 * i + a - 4) * 64 + p] = s;
+        for (int ax = 0; ax < 3; ax++)
+#pragma unroll
+            for (int k = 0; k < 6; k++) c[ax][k] = C[(ax * 6 + k) * 3];
+#pragma unroll
+        for (int a = 1; a < 10; a++) {
+            double s = 0.0;
+#pragma unroll
+            for (int ax = 0; ax < 3; ax++) s += b[ax][a_kx(a)] * c[ax][a_kk(a)];
+            if (a < 4 && f == 0) {
+                if (g.periodic) s += g.pp[3 * i + a - 1];
+                if (i == a - 1) s += 1.0;
+            }
+            u[f][a - 1] = s;
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < 9; a++) {
+        double v0 = u[0][a];
+        if constexpr (NR == 2) {
+            v0 = R.r00 * v0 + R.r01 * u[NR - 1][a];
+            S.pt[(a < 3 ? A::F + 9 + 3 * i + a : A::G + 18 + 6 * i + a - 3) * 64 + p] = R.r11 * u[NR - 1][a];
+        }
+        S.pt[(a < 3 ? A::F + 3 * i + a : A::G + 6 * i + a - 3) * 64 + p] = v0;
     }
 }
-/* strains and stresses: warps 0-1 the strain part (CN, S), warps 2-7 TAU for one K each */
-__device__ __forceinline__ void sf_point_data(sf_smem &S, const igab_geom &g, const sf_elem &E, int buf, int tid)
+/* CN_IJ (the normal strains' Hessian from those of (vvol, va, vb)) times w */
+__device__ __forceinline__ void sf_store_cn(double *cn, double w, double h0, double haa, double hbb, double hab)
 {
+    const double a0 = h0 * (1.0 / 3.0), a1 = haa * 0.5, a2 = hbb * (1.0 / 6.0),
+                 a3 = hab * (IGAB_INV_SQRT2 * IGAB_INV_SQRT6);
+    cn[0 * 64] = w * (a0 + a1 + a2 + 2.0 * a3);
+    cn[1 * 64] = w * (a0 - a1 + a2);
+    cn[2 * 64] = w * (a0 - 2.0 * a2 - 2.0 * a3);
+    cn[3 * 64] = w * (a0 + a1 + a2 - 2.0 * a3);
+    cn[4 * 64] = w * (a0 - 2.0 * a2 + 2.0 * a3);
+    cn[5 * 64] = w * (a0 + 4.0 * a2);
+}
+/* strains and stresses: warps 0-1 the strain part (CN, S), warps 2-7 TAU for one K each */
+template <int NR>
+__device__ __forceinline__ void sf_point_data(sf_smem<NR> &S, const igab_geom &g, const sf_coef &R, int buf, int tid)
+{
+    using A = pt_at<NR>;
     const int p = tid & 63, qz = p & 3, qy = (p >> 2) & 3, qx = p >> 4;
     double *pt = S.pt + p;
     const double w = S.wh[buf][0][qx] * S.wh[buf][1][qy] * S.wh[buf][2][qz] * S.esc[buf];
-    double F[3][3];
+    double F[NR][3][3];
 #pragma unroll
-    for (int k = 0; k < 3; k++)
+    for (int r = 0; r < NR; r++)
 #pragma unroll
-        for (int J = 0; J < 3; J++) F[k][J] = pt[(P_F + 3 * k + J) * 64];
+        for (int k = 0; k < 3; k++)
+#pragma unroll
+            for (int J = 0; J < 3; J++) F[r][k][J] = pt[(A::F + 9 * r + 3 * k + J) * 64];
     if (tid < 64) {
         const double is2 = IGAB_INV_SQRT2, is3 = IGAB_INV_SQRT3, is6 = IGAB_INV_SQRT6;
-        double e[6];
+        const double c36 = g.coef.c36, c37 = g.coef.c37, c38 = g.coef.c38, p3 = g.coef.p3;
+        pt[A::W * 64] = w;
+        double sv, sa, sb, sh[3];   /* Phi' of (vvol, va, vb) and the shear stresses E_01, E_02, E_12 */
+        if constexpr (NR == 1) {
+            double e[6];
 #pragma unroll
-        for (int c = 0; c < 6; c++) {
-            const int I = s_i(c), J = s_k(c);
-            e[c] = 0.5 * (F[0][I] * F[0][J] + F[1][I] * F[1][J] + F[2][I] * F[2][J] - (I == J ? 1.0 : 0.0));
+            for (int c = 0; c < 6; c++) {
+                const int I = s_i(c), J = s_k(c);
+                e[c] = 0.5 * (F[0][0][I] * F[0][0][J] + F[0][1][I] * F[0][1][J] + F[0][2][I] * F[0][2][J] -
+                              (I == J ? 1.0 : 0.0));
+            }
+            const double vv = (e[0] + e[3] + e[5]) * is3, va = (e[0] - e[3]) * is2,
+                         vb = (e[0] + e[3] - 2.0 * e[5]) * is6;
+            const double s2 = va * va + vb * vb;
+            sv = 2.0 * g.coef.p2 * vv;
+            sa = -6.0 * c36 * va * vb + 2.0 * c37 * va + 4.0 * c38 * s2 * va;
+            sb = 3.0 * c36 * (vb * vb - va * va) + 2.0 * c37 * vb + 4.0 * c38 * s2 * vb;
+            const double haa = -6.0 * c36 * vb + 2.0 * c37 + 4.0 * c38 * (3.0 * va * va + vb * vb);
+            const double hbb = 6.0 * c36 * vb + 2.0 * c37 + 4.0 * c38 * (va * va + 3.0 * vb * vb);
+            const double hab = -6.0 * c36 * va + 8.0 * c38 * va * vb;
+            sf_store_cn(pt + A::CN * 64, w, 2.0 * g.coef.p2, haa, hbb, hab);
+            sh[0] = e[1]; sh[1] = e[2]; sh[2] = e[4];
+        } else {
+            /* E(s) = E0 + s E1 + s^2 E2 along u(s) = m + s h, from F0 = al F^0 + be F^1, F1 = ga F^1 */
+            igab_tay<4> v[3];
+            double e[3][3];
+#pragma unroll
+            for (int I = 0; I < 3; I++) {
+                double x0 = 0.0, x1 = 0.0, x2 = 0.0;
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    const double a = R.al * F[0][k][I] + R.be * F[NR - 1][k][I], b = R.ga * F[NR - 1][k][I];
+                    x0 += a * a;
+                    x1 += a * b;
+                    x2 += b * b;
+                }
+                e[0][I] = 0.5 * (x0 - 1.0);
+                e[1][I] = x1;
+                e[2][I] = 0.5 * x2;
+            }
+#pragma unroll
+            for (int j = 0; j < 3; j++) {
+                v[0].c[j] = (e[j][0] + e[j][1] + e[j][2]) * is3;
+                v[1].c[j] = (e[j][0] - e[j][1]) * is2;
+                v[2].c[j] = (e[j][0] + e[j][1] - 2.0 * e[j][2]) * is6;
+            }
+            v[0].c[3] = v[1].c[3] = v[2].c[3] = 0.0;
+            const igab_tay<4> aa = v[1] * v[1], bb = v[2] * v[2], ab = v[1] * v[2], s2 = aa + bb;
+            const igab_tay<4> sa3 = s2 * v[1], sb3 = s2 * v[2];
+            sv = sa = sb = 0.0;
+            /* N_j = sum_b tw[j + b] f_b of the parts of Phi'' that vary along s; the constant part is the same
+             * in both hat fields and does not couple them */
+            double na[3] = {0.0, 0.0, 0.0}, nb[3] = {0.0, 0.0, 0.0}, nab[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+            for (int b = 0; b < 4; b++) {
+                const double fa = -6.0 * c36 * v[2].c[b] + 4.0 * c38 * (3.0 * aa.c[b] + bb.c[b]);
+                const double fb = 6.0 * c36 * v[2].c[b] + 4.0 * c38 * (aa.c[b] + 3.0 * bb.c[b]);
+                const double fab = -6.0 * c36 * v[1].c[b] + 8.0 * c38 * ab.c[b];
+                sv += g.tw[b] * (2.0 * g.coef.p2 * v[0].c[b]);
+                sa += g.tw[b] * (-6.0 * c36 * ab.c[b] + 2.0 * c37 * v[1].c[b] + 4.0 * c38 * sa3.c[b]);
+                sb += g.tw[b] * (3.0 * c36 * (bb.c[b] - aa.c[b]) + 2.0 * c37 * v[2].c[b] + 4.0 * c38 * sb3.c[b]);
+#pragma unroll
+                for (int j = 0; j < 3; j++)
+                    if (j + b < 4) {
+                        na[j] += g.tw[j + b] * fa;
+                        nb[j] += g.tw[j + b] * fb;
+                        nab[j] += g.tw[j + b] * fab;
+                    }
+            }
+            const double q00 = R.al * R.al, q01a = R.al * R.be, q01b = R.al * R.ga, q11a = R.be * R.be,
+                         q11b = 2.0 * R.be * R.ga, q11c = R.ga * R.ga, h0 = 2.0 * g.coef.p2, hc = 2.0 * c37;
+            double *cn = pt + A::CN * 64;
+            sf_store_cn(cn, w, h0, hc + q00 * na[0], hc + q00 * nb[0], q00 * nab[0]);
+            sf_store_cn(cn + 6 * 64, w, 0.0, q01a * na[0] + q01b * na[1], q01a * nb[0] + q01b * nb[1],
+                        q01a * nab[0] + q01b * nab[1]);
+            sf_store_cn(cn + 12 * 64, w, h0, hc + q11a * na[0] + q11b * na[1] + q11c * na[2],
+                        hc + q11a * nb[0] + q11b * nb[1] + q11c * nb[2],
+                        q11a * nab[0] + q11b * nab[1] + q11c * nab[2]);
+            sh[0] = sh[1] = sh[2] = 0.0;
+#pragma unroll
+            for (int r = 0; r < NR; r++)
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    sh[0] += 0.5 * F[r][k][0] * F[r][k][1];
+                    sh[1] += 0.5 * F[r][k][0] * F[r][k][2];
+                    sh[2] += 0.5 * F[r][k][1] * F[r][k][2];
+                }
         }
-        const double vv = (e[0] + e[3] + e[5]) * is3, va = (e[0] - e[3]) * is2, vb = (e[0] + e[3] - 2.0 * e[5]) * is6;
-        const double c36 = g.coef.c36, c37 = g.coef.c37, c38 = g.coef.c38;
-        const double s2 = va * va + vb * vb;
-        const double d0 = 2.0 * g.coef.p2 * vv;
-        const double da = -6.0 * c36 * va * vb + 2.0 * c37 * va + 4.0 * c38 * s2 * va;
-        const double db = 3.0 * c36 * (vb * vb - va * va) + 2.0 * c37 * vb + 4.0 * c38 * s2 * vb;
-        const double h0 = 2.0 * g.coef.p2;
-        const double haa = -6.0 * c36 * vb + 2.0 * c37 + 4.0 * c38 * (3.0 * va * va + vb * vb);
-        const double hbb = 6.0 * c36 * vb + 2.0 * c37 + 4.0 * c38 * (va * va + 3.0 * vb * vb);
-        const double hab = -6.0 * c36 * va + 8.0 * c38 * va * vb;
-        /* CN_IJ = d2 Phi / dE_II dE_JJ through (vvol, va, vb) */
-        const double a0 = h0 * (1.0 / 3.0), a1 = haa * 0.5, a2 = hbb * (1.0 / 6.0), a3 = hab * (is2 * is6);
-        pt[P_W * 64] = w;
-        pt[(P_CN + 0) * 64] = w * (a0 + a1 + a2 + 2.0 * a3);
-        pt[(P_CN + 1) * 64] = w * (a0 - a1 + a2);
-        pt[(P_CN + 2) * 64] = w * (a0 - 2.0 * a2 - 2.0 * a3);
-        pt[(P_CN + 3) * 64] = w * (a0 + a1 + a2 - 2.0 * a3);
-        pt[(P_CN + 4) * 64] = w * (a0 - 2.0 * a2 + 2.0 * a3);
-        pt[(P_CN + 5) * 64] = w * (a0 + 4.0 * a2);
-        pt[(P_S + 0) * 64] = w * (d0 * is3 + da * is2 + db * is6);
-        pt[(P_S + 3) * 64] = w * (d0 * is3 - da * is2 + db * is6);
-        pt[(P_S + 5) * 64] = w * (d0 * is3 - 2.0 * db * is6);
-        pt[(P_S + 1) * 64] = w * g.coef.p3 * e[1];
-        pt[(P_S + 2) * 64] = w * g.coef.p3 * e[2];
-        pt[(P_S + 4) * 64] = w * g.coef.p3 * e[4];
+        pt[(A::S + 0) * 64] = w * (sv * is3 + sa * is2 + sb * is6);
+        pt[(A::S + 3) * 64] = w * (sv * is3 - sa * is2 + sb * is6);
+        pt[(A::S + 5) * 64] = w * (sv * is3 - 2.0 * sb * is6);
+        pt[(A::S + 1) * 64] = w * p3 * sh[0];
+        pt[(A::S + 2) * 64] = w * p3 * sh[1];
+        pt[(A::S + 4) * 64] = w * p3 * sh[2];
     } else {
         const int K = (tid >> 6) - 1;
-        double ek[3];
+        double ek[3] = {0.0, 0.0, 0.0};
 #pragma unroll
-        for (int I = 0; I < 3; I++) {
-            const int c = igab_idx6(I, K);
-            ek[I] = F[0][I] * pt[(P_G + c) * 64] + F[1][I] * pt[(P_G + 6 + c) * 64] + F[2][I] * pt[(P_G + 12 + c) * 64];
-        }
+        for (int r = 0; r < NR; r++)
+#pragma unroll
+            for (int I = 0; I < 3; I++) {
+                const double *G = pt + (A::G + 18 * r + igab_idx6(I, K)) * 64;
+                ek[I] += F[r][0][I] * G[0] + F[r][1][I] * G[6 * 64] + F[r][2][I] * G[12 * 64];
+            }
         const double m = (ek[0] + ek[1] + ek[2]) * (1.0 / 3.0), wa = w * 2.0 * g.coef.p4sq;
 #pragma unroll
-        for (int I = 0; I < 3; I++) pt[(P_TAU + 3 * I + K) * 64] = wa * (ek[I] - m);
+        for (int I = 0; I < 3; I++) pt[(A::TAU + 3 * I + K) * 64] = wa * (ek[I] - m);
     }
-    if (tid < 27) {
-        sf_row &R = S.row[tid];
-        elem_row_base(g, E.ex, E.ey, E.ez, 3 * tid, R.rb, R.rsx, R.rsy);
-        const int x = E.ex + tid / 9;
-        const int x0 = x > 2 ? x - 2 : 0, x1 = x + 2 < g.nb[0] - 1 ? x + 2 : g.nb[0] - 1;
-        R.len = (x1 - x0 + 1) * R.rsx;
-    }
+}
+/* where the rows (a, k) of the element lie in the CSR values */
+template <int NR>
+__device__ __forceinline__ void sf_rows(sf_smem<NR> &S, const igab_geom &g, const sf_elem &E, int tid)
+{
+    if (tid >= 81) return;
+    sf_row R;
+    elem_row_base(g, E.ex, E.ey, E.ez, 3 * (tid % 27) + tid / 27, R.rb, R.rsx, R.rsy);
+    (&S.row[0][0])[tid] = R;
 }
 
 /* the element of a tile at or after position le (8: none), le = 4 dx + 2 dy + dz */
@@ -558,98 +772,96 @@ __device__ __forceinline__ int sf_next(const tile_t &T, int le)
     return le;
 }
 
-template <typename T>
-__device__ __forceinline__ void sf_tile(const igab_geom &g, const tile_t &Tl, const double *__restrict__ U,
-                                        T *__restrict__ vals, sf_smem &S)
+template <typename T, int NR>
+__device__ __forceinline__ void sf_tile(const igab_geom &g, const sf_coef &C, const tile_t &Tl,
+                                        const double *__restrict__ U, T *__restrict__ vals, sf_smem<NR> &S)
 {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const double aon = g.coef.p4sq * (4.0 / 3.0), aoff = g.coef.p4sq * (-2.0 / 3.0), ash = g.coef.p3 * 0.5;
     int le = sf_next(Tl, 0), buf = 0;
     sf_elem E = {Tl.e0[0] + (le >> 2), Tl.e0[1] + ((le >> 1) & 1), Tl.e0[2] + (le & 1)};
-    sf_stage(S, sf_prefetch(g, U, E, tid), buf, tid);
+    sf_load<NR>(S, g, U, E, buf, tid);
+    sf_copy_wait();
     __syncthreads();
-    sf_interp_z(S, buf, tid);
+    sf_interp_z<NR>(S, buf, tid);
     __syncthreads();
-    sf_interp_y(S, buf, tid);
+    sf_interp_y<NR>(S, buf, tid);
     __syncthreads();
-    sf_interp_x(S, g, buf, tid);
+    sf_interp_x<NR>(S, g, C, buf, tid);
     __syncthreads();
-    sf_point_data(S, g, E, buf, tid);
+    sf_point_data<NR>(S, g, C, buf, tid);
     __syncthreads();
 
-#define SF_S1_(DG, k, l)                                                                              \
-    switch (warp >> 1) {                                                                              \
-    case 0: sf_s1<0, DG>(S, S.tab[buf][2], lane, warp & 1, k, l, aon, aoff, ash); break;              \
-    case 1: sf_s1<1, DG>(S, S.tab[buf][2], lane, warp & 1, k, l, aon, aoff, ash); break;              \
-    case 2: sf_s1<2, DG>(S, S.tab[buf][2], lane, warp & 1, k, l, aon, aoff, ash); break;              \
-    default: sf_s1<3, DG>(S, S.tab[buf][2], lane, warp & 1, k, l, aon, aoff, ash); break;             \
+#define SF_S1_(DG, k, l)                                                             \
+    switch (warp >> 1) {                                                             \
+    case 0: sf_s1<NR, 0, DG>(S, tab[2], lane, warp & 1, k, l, C); break;             \
+    case 1: sf_s1<NR, 1, DG>(S, tab[2], lane, warp & 1, k, l, C); break;             \
+    case 2: sf_s1<NR, 2, DG>(S, tab[2], lane, warp & 1, k, l, C); break;             \
+    default: sf_s1<NR, 3, DG>(S, tab[2], lane, warp & 1, k, l, C); break;            \
     }
-#define SF_S2_(DG)                                                                                    \
-    if (warp < 4) sf_s2<0, DG>(S, S.tab[buf][1], lane, warp & 3);                                     \
-    else sf_s2<1, DG>(S, S.tab[buf][1], lane, warp & 3);
+#define SF_S2_(DG)                                                                   \
+    if (warp < 4) sf_s2<NR, 0, DG>(S, tab[1], lane, warp & 3);                       \
+    else sf_s2<NR, 1, DG>(S, tab[1], lane, warp & 3);
 
     while (true) {
         const int ln = sf_next(Tl, le + 1);
-        double pre = 0.0;
-        sf_elem En = E;
+        const sf_elem En = {Tl.e0[0] + (ln >> 2), Tl.e0[1] + ((ln >> 1) & 1), Tl.e0[2] + (ln & 1)};
+        const double(*tab)[IGAB_TAB1D] = S.tab[buf];
         /* pairs in the order (0,0) (0,1) (0,2) (1,1) (1,2) (2,2), slots 0 1 2 3 0 4 */
         for (int p = 0; p < 6; p++) {
             const int k = p < 3 ? 0 : (p < 5 ? 1 : 2), l = p < 3 ? p : (p < 5 ? p - 2 : 2);
             const bool dg = k == l;
             if (p > 0) {
                 double *Ks = SF_KSLOT(S, p == 5 ? 0 : p - 1);
-                if (p == 1 || p == 4) sf_s3<true>(S, S.tab[buf][0], Ks, warp, lane);
-                else sf_s3<false>(S, S.tab[buf][0], Ks, warp, lane);
+                if (p == 1 || p == 4) sf_s3_all<NR, true>(S, tab[0], Ks, warp, lane);
+                else sf_s3_all<NR, false>(S, tab[0], Ks, warp, lane);
             }
             if (dg) { SF_S1_(true, k, l) } else { SF_S1_(false, k, l) }
-            if (p == 4) sf_fix_x(S, 0, 1, 2, 3, tid);
+            if (p == 4) sf_fix_x<NR>(S, 0, 1, 2, 3, tid);
             __syncthreads();
             if (dg) { SF_S2_(true) } else { SF_S2_(false) }
-            if (p == 3) sf_fix_zy(S, 0, 1, 2, 3, warp, lane);
-            if (p == 4) sf_scatter<T>(S, vals, 0, 0, 1, 2, tid);
-            if (p == 5) {
-                sf_fix_zy(S, 3, 0, 0, 2, warp, lane);
-                if (ln < 8) {
-                    En = {Tl.e0[0] + (ln >> 2), Tl.e0[1] + ((ln >> 1) & 1), Tl.e0[2] + (ln & 1)};
-                    pre = sf_prefetch(g, U, En, tid);
-                }
-            }
+            if (p == 0) sf_rows<NR>(S, g, E, tid);
+            if (p == 3) sf_fix_zy<NR>(S, 0, 1, 2, 3, warp, lane);
+            if (p == 4) sf_scatter<T, NR>(S, vals, 0, 0, 1, 2, tid);
+            if (p == 5) sf_fix_zy<NR>(S, 3, 0, 0, 2, warp, lane);
             __syncthreads();
         }
-        sf_s3<true>(S, S.tab[buf][0], SF_KSLOT(S, 4), warp, lane);
-        sf_fix_x(S, 3, 0, 0, 2, tid);
-        if (ln < 8) sf_stage(S, pre, buf ^ 1, tid);
+        if (ln < 8) sf_load<NR>(S, g, U, En, buf ^ 1, tid);
+        sf_s3_all<NR, true>(S, tab[0], SF_KSLOT(S, 4), warp, lane);
+        sf_fix_x<NR>(S, 3, 0, 0, 2, tid);
+        sf_copy_wait();
         __syncthreads();
-        sf_fix_zy(S, 4, 4, 4, 1, warp, lane);
-        sf_scatter<T>(S, vals, 1, 1, 3, 0, tid);
-        if (ln < 8) sf_interp_z(S, buf ^ 1, tid);
+        sf_fix_zy<NR>(S, 4, 4, 4, 1, warp, lane);
+        sf_scatter<T, NR>(S, vals, 1, 1, 3, 0, tid);
+        if (ln < 8) sf_interp_z<NR>(S, buf ^ 1, tid);
         __syncthreads();
-        sf_fix_x(S, 4, 4, 4, 1, tid);
-        if (ln < 8) sf_interp_y(S, buf ^ 1, tid);
+        sf_fix_x<NR>(S, 4, 4, 4, 1, tid);
+        if (ln < 8) sf_interp_y<NR>(S, buf ^ 1, tid);
         __syncthreads();
-        sf_scatter<T>(S, vals, 2, 2, 0, 4, tid);
-        if (ln < 8) sf_interp_x(S, g, buf ^ 1, tid);
+        sf_scatter<T, NR>(S, vals, 2, 2, 0, 4, tid);
+        if (ln < 8) sf_interp_x<NR>(S, g, C, buf ^ 1, tid);
         __syncthreads();
         if (ln >= 8) break;
         buf ^= 1;
         le = ln;
         E = En;
-        sf_point_data(S, g, E, buf, tid);
+        sf_point_data<NR>(S, g, C, buf, tid);
         __syncthreads();
     }
 #undef SF_S1_
 #undef SF_S2_
 }
 
-template <typename T>
-__global__ void __launch_bounds__(SF_THR, 2) k_tan_sf(igab_geom g, const double *__restrict__ U, T *__restrict__ vals,
-                                                      int colour, int tile0)
+/* two blocks per SM for phys/ge; the transient point data (45 KB) and its registers leave room for one */
+template <typename T, int NR>
+__global__ void __launch_bounds__(SF_THR, NR == 1 ? 2 : 1) k_tan_sf(igab_geom g, sf_coef C,
+                                                                    const double *__restrict__ U,
+                                                                    T *__restrict__ vals, int colour, int tile0)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    sf_smem &S = *reinterpret_cast<sf_smem *>(smem_raw);
+    sf_smem<NR> &S = *reinterpret_cast<sf_smem<NR> *>(smem_raw);
     tile_t Tl;
     if (!decode_tile(g, SF_TE, colour, tile0 + blockIdx.x, Tl)) return;
-    sf_tile<T>(g, Tl, U, vals, S);
+    sf_tile<T, NR>(g, C, Tl, U, vals, S);
 }
 
 /* persistent over the tiles of every instance of a batch */
@@ -658,28 +870,28 @@ __global__ void __launch_bounds__(SF_THR, 2) k_tan_sf_batch(igab_batch_dev B, co
                                                             T *__restrict__ vals)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    sf_smem &S = *reinterpret_cast<sf_smem *>(smem_raw);
+    sf_smem<1> &S = *reinterpret_cast<sf_smem<1> *>(smem_raw);
     __shared__ batch_slot sl;
     while (batch_next(B, sl)) {
         tile_t Tl;
         decode_tile(sl.g, SF_TE, sl.colour, sl.tile, Tl);
-        sf_tile<T>(sl.g, Tl, U + B.dof_off[sl.inst], vals + B.nnz_off[sl.inst], S);
+        const sf_coef C = sf_coef_ge(sl.g);
+        sf_tile<T, 1>(sl.g, C, Tl, U + B.dof_off[sl.inst], vals + B.nnz_off[sl.inst], S);
         batch_done(B, sl);
     }
 }
 
-template <typename T>
-int launch_sf(igab_ctx *c, const double *dU, T *dv, int tx0, int tx1)
+template <typename T, int NR>
+int launch_sf(igab_ctx *c, const igab_geom &g, const sf_coef &C, const double *dU, T *dv, int tx0, int tx1)
 {
-    const igab_geom g = c->geom();
-    const size_t sm = sizeof(sf_smem);
-    IGAB_CUDA_TRY(cudaFuncSetAttribute(k_tan_sf<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    const size_t sm = sizeof(sf_smem<NR>);
+    IGAB_CUDA_TRY(cudaFuncSetAttribute(k_tan_sf<T, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     for (int k = 0; k < 8; k++) {
         const int colour = igab_colour_at(c->colour_order, k);
         long first = 0;
         const long nt = tiles_of_colour_in(g, SF_TE, colour, tx0, tx1, &first);
         if (nt == 0) continue;
-        k_tan_sf<T><<<(unsigned)nt, SF_THR, sm, c->stream>>>(g, dU, dv, colour, (int)first);
+        k_tan_sf<T, NR><<<(unsigned)nt, SF_THR, sm, c->stream>>>(g, C, dU, dv, colour, (int)first);
         c->last_launches++;
     }
     IGAB_CUDA_TRY(cudaGetLastError());
@@ -690,14 +902,41 @@ int launch_sf(igab_ctx *c, const double *dU, T *dv, int tx0, int tx1)
 
 int igab_launch_tan_sf(igab_ctx *c, const double *dU, void *dv, int prec, int tx0, int tx1)
 {
-    return prec == IGAB_PREC_FP64 ? launch_sf<double>(c, dU, (double *)dv, tx0, tx1)
-                                  : launch_sf<float>(c, dU, (float *)dv, tx0, tx1);
+    const igab_geom g = c->geom();
+    if (c->phys == IGAB_PHYS_GETIME) return igab_launch_tan_getime_level(c, dU, dv, prec, 0, tx0, tx1);
+    const sf_coef C = sf_coef_ge(g);
+    return prec == IGAB_PREC_FP64 ? launch_sf<double, 1>(c, g, C, dU, (double *)dv, tx0, tx1)
+                                  : launch_sf<float, 1>(c, g, C, dU, (float *)dv, tx0, tx1);
+}
+
+int igab_launch_tan_getime_level(igab_ctx *c, const double *dU, void *dv, int prec, int level, int tx0, int tx1)
+{
+    igab_geom g = c->geom();
+    if (level == 1) {          /* d r / d u1 */
+        const double w[4] = {0.5, 0.25, 1.0 / 6.0, 0.125};
+        for (int j = 0; j < 4; j++) g.tw[j] = w[j];
+        g.tmass = -2.0 * g.rho / (g.dt * g.dt);
+    } else if (level == 2) {   /* d r / d u0 */
+        const double w[4] = {0.25, 1.0 / 12.0, 1.0 / 24.0, 0.125};
+        for (int j = 0; j < 4; j++) g.tw[j] = w[j];
+        g.tmass = g.rho / (g.dt * g.dt) - g.cii / (2.0 * g.dt);
+    }
+    sf_coef C = sf_coef_ge(g);
+    C.mass = g.tmass;
+    C.r00 = sqrt(g.tw[0]);
+    C.r01 = g.tw[1] / C.r00;
+    C.r11 = sqrt(g.tw[2] - C.r01 * C.r01);
+    C.al = 1.0 / C.r00;
+    C.ga = 1.0 / C.r11;
+    C.be = -C.r01 * C.al * C.ga;
+    return prec == IGAB_PREC_FP64 ? launch_sf<double, 2>(c, g, C, dU, (double *)dv, tx0, tx1)
+                                  : launch_sf<float, 2>(c, g, C, dU, (float *)dv, tx0, tx1);
 }
 
 template <typename T>
 static int launch_sf_batch(const igab_batch_dev &B, int grid, cudaStream_t st, const double *dU, T *dv)
 {
-    const size_t sm = sizeof(sf_smem);
+    const size_t sm = sizeof(sf_smem<1>);
     IGAB_CUDA_TRY(cudaFuncSetAttribute(k_tan_sf_batch<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     k_tan_sf_batch<T><<<grid, SF_THR, sm, st>>>(B, dU, dv);
     IGAB_CUDA_TRY(cudaGetLastError());
@@ -713,7 +952,7 @@ int igab_launch_tan_sf_batch(const igab_batch_dev &B, int grid, cudaStream_t st,
 template <typename T>
 static int occupancy_sf(int *per_sm)
 {
-    const size_t sm = sizeof(sf_smem);
+    const size_t sm = sizeof(sf_smem<1>);
     IGAB_CUDA_TRY(cudaFuncSetAttribute(k_tan_sf_batch<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     IGAB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_tan_sf_batch<T>, SF_THR, sm));
     return 0;
