@@ -337,6 +337,53 @@ static int build_neumann(igab_ctx *c)
     return 0;
 }
 
+static int is_capturing(cudaStream_t s, bool *yes)
+{
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    *yes = false;
+    if (!s) return 0;   /* the legacy stream cannot be captured */
+    IGAB_CUDA_TRY(cudaStreamIsCapturing(s, &st));
+    *yes = st != cudaStreamCaptureStatusNone;
+    return 0;
+}
+
+int igab_scratch_order(igab_ctx *c)
+{
+    if (c->scratch_ev && c->scratch_stream != c->stream)
+        IGAB_CUDA_TRY(cudaStreamWaitEvent(c->stream, c->scratch_ev, 0));
+    c->scratch_stream = c->stream;
+    return 0;
+}
+
+int igab_scratch_used(igab_ctx *c)
+{
+    if (c->own_capture || (!c->d_scratch[0] && !c->d_scratch[1])) return 0;
+    if (!c->scratch_ev) IGAB_CUDA_TRY(cudaEventCreateWithFlags(&c->scratch_ev, cudaEventDisableTiming));
+    IGAB_CUDA_TRY(cudaEventRecord(c->scratch_ev, c->stream));
+    c->scratch_stream = c->stream;
+    return 0;
+}
+
+int igab_scratch(igab_ctx *c, int kind, size_t bytes, double **out)
+{
+    *out = nullptr;
+    bool cap = false;
+    int rc = is_capturing(c->stream, &cap);
+    if (rc) return rc;
+    if (cap && !c->own_capture) return 0;
+    if (!c->d_scratch[kind]) {
+        if (cap) return 0;
+        if (cudaMalloc((void **)&c->d_scratch[kind], bytes) != cudaSuccess) {
+            cudaGetLastError();
+            c->d_scratch[kind] = nullptr;
+            return 0;
+        }
+    }
+    if (!cap && (rc = igab_scratch_order(c))) return rc;
+    *out = c->d_scratch[kind];
+    return 0;
+}
+
 static void free_ctx(igab_ctx *c)
 {
     for (int d = 0; d < 3; d++) {
@@ -348,6 +395,8 @@ static void free_ctx(igab_ctx *c)
     cudaFree(c->d_U); cudaFree(c->d_R); cudaFree(c->d_vals);
     cudaFree(c->d_escale); cudaFree(c->d_lam); cudaFree(c->d_status);
     cudaFree(c->d_dens_part); cudaFree(c->d_HH);
+    cudaFree(c->d_scratch[0]); cudaFree(c->d_scratch[1]);
+    if (c->scratch_ev) cudaEventDestroy(c->scratch_ev);
     igab_periodic_release(c);
     igab_krylov_release(c);
     igab_newton_release(c);
@@ -832,9 +881,7 @@ extern "C" int igab_history_jacobian_device(igab_ctx *ctx, const double *U_dev, 
     ARG_CHECK(prec == IGAB_PREC_FP64 || prec == IGAB_PREC_FP32, "igab_history_jacobian_device: bad precision");
     IGAB_CUDA_TRY(cudaSetDevice(ctx->device));
     ctx->last_launches = 0;
-    const size_t es = prec == IGAB_PREC_FP64 ? sizeof(double) : sizeof(float);
-    IGAB_CUDA_TRY(cudaMemsetAsync(vals_dev, 0, (size_t)ctx->nnz * es, ctx->stream));
-    int rc = igab_launch_tan_getime_level(ctx, U_dev, vals_dev, prec, level, 0, (ctx->ne[0] + 1) / 2);
+    int rc = igab_launch_tan_getime_level(ctx, U_dev, vals_dev, prec, level, 0, (ctx->ne[0] + 1) / 2, true);
     if (!rc) rc = igab_launch_zero_csr_rows(ctx, vals_dev, prec);
     return rc;
 }
@@ -1120,8 +1167,10 @@ extern "C" int igab_graph_capture(igab_ctx *ctx, const double *U_dev, double *R_
         if (e != cudaSuccess) { igab_set_error("cudaStreamBeginCapture: %s", cudaGetErrorString(e)); rc = IGAB_ERR_CUDA; }
         else {
             int rc2 = 0;
+            ctx->own_capture = true;
             if (what & 1) rc2 = igab_launch_residual(ctx, U_dev, R_dev);
             if (!rc2 && (what & 2)) rc2 = igab_launch_tangent(ctx, U_dev, vals_dev, prec);
+            ctx->own_capture = false;
             cudaGraph_t gr = nullptr;
             e = cudaStreamEndCapture(ctx->stream, &gr);
             if (rc2) { rc = rc2; if (gr) cudaGraphDestroy(gr); }
@@ -1142,8 +1191,10 @@ extern "C" int igab_graph_launch(igab_ctx *ctx)
 {
     ARG_CHECK(ctx && ctx->graph_exec, "igab_graph_launch: no captured graph");
     IGAB_CUDA_TRY(cudaSetDevice(ctx->device));
+    int rc = igab_scratch_order(ctx);
+    if (rc) return rc;
     IGAB_CUDA_TRY(cudaGraphLaunch(ctx->graph_exec, ctx->stream));
-    return 0;
+    return igab_scratch_used(ctx);
 }
 
 /* ------------------------------------------------------------------ adjoint */

@@ -100,6 +100,15 @@ __device__ __forceinline__ void elem_row_base(const igab_geom &g, int ex, int ey
     rsy = nzb * 3;
 }
 
+/* the elements [a, b) of one direction (at most three) split into those of even and of odd tiles of two: at most
+ * two each, consecutive, [lo[parity], hi[parity]) */
+__device__ __forceinline__ void elem_parity_ranges(int a, int b, int lo[2], int hi[2])
+{
+    const int m = min(b, 2 * (a >> 1) + 2), odd = (a >> 1) & 1;
+    lo[0] = odd ? m : a; hi[0] = odd ? b : m;
+    lo[1] = odd ? a : m; hi[1] = odd ? m : b;
+}
+
 /* per-element integrand scale (1 when no scaling is set) */
 __device__ __forceinline__ double elem_scale(const igab_geom &g, int ex, int ey, int ez)
 {

@@ -162,6 +162,12 @@ struct igab_ctx {
     int periodic[3] = {0, 0, 0};
     struct igab_periodic *per = nullptr;
 
+    /* scratch of the assembly (igab_scratch) */
+    double *d_scratch[2] = {nullptr, nullptr};
+    cudaEvent_t scratch_ev = nullptr;      /* after its last use, on scratch_stream */
+    cudaStream_t scratch_stream = nullptr;
+    bool own_capture = false;              /* the context itself captures its stream */
+
     /* captured assembly graph */
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graph_exec = nullptr;
@@ -224,7 +230,8 @@ int igab_launch_basis_tables(igab_ctx *c, int d, const double *dkv, const double
 int igab_launch_fma_peak(int prec, double *tflops);
 int igab_launch_dmma_peak(double *tflops);   /* igab_probes.cu */
 /* tangent volume kernels over the tiles with x tile coordinate in [tx0, tx1) (tiles of 2 elements) */
-int igab_launch_tan_sf(igab_ctx *c, const double *dU, void *dv, int prec, int tx0, int tx1);   /* igab_tangent_sf.cu */
+/* igab_tangent_sf.cu; zero: clear the values first (where the kernels add to them) */
+int igab_launch_tan_sf(igab_ctx *c, const double *dU, void *dv, int prec, int tx0, int tx1, bool zero);
 /* persistent batched launches (igab_batch.cu builds the work list) */
 int igab_launch_res_batch(const igab_batch_dev &B, int grid, cudaStream_t s, const double *dU, double *dR);
 int igab_launch_tan_sf_batch(const igab_batch_dev &B, int grid, cudaStream_t s, const double *dU, void *dv, int prec);
@@ -239,7 +246,16 @@ int igab_batch_occupancy_tan(int prec, int *per_sm);
 /* zero the Dirichlet rows of CSR values (rows only) */
 int igab_launch_zero_csr_rows(igab_ctx *c, void *dv, int prec);
 /* the transient tangent (level 0) or history Jacobian (level 1, 2), x tiles [tx0, tx1) */
-int igab_launch_tan_getime_level(igab_ctx *c, const double *dU, void *dv, int prec, int level, int tx0, int tx1);
+int igab_launch_tan_getime_level(igab_ctx *c, const double *dU, void *dv, int prec, int level, int tx0, int tx1,
+                                 bool zero);
+/* Scratch arrays of the assembly (igab_capi.cu), allocated on first use and kept by the context.  *out stays null
+ * (the caller takes its stateless path) when there is no memory, or while somebody else captures the stream: such
+ * a graph could be replayed beside other work of the context.  Uses on different streams are ordered by an event
+ * that igab_scratch_used records; igab_scratch_order is the wait alone, before a graph replay. */
+enum igab_scratch_kind { IGAB_SCRATCH_TAN = 0, IGAB_SCRATCH_RES = 1 };
+int igab_scratch(igab_ctx *c, int kind, size_t bytes, double **out);
+int igab_scratch_used(igab_ctx *c);
+int igab_scratch_order(igab_ctx *c);
 int igab_launch_exp_scale(igab_ctx *c, const double *dg);
 int igab_launch_adjoint_dRdg(igab_ctx *c, const double *dU, const double *dlam, double *dgrad);
 int igab_launch_tangent_transpose(igab_ctx *c, const void *dvals, int prec, const double *dx, double *dy);

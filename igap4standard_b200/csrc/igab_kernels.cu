@@ -865,12 +865,16 @@ int launch_tan_volume(igab_ctx *c, const igab_geom &g, const double *dU, T *dv)
 }
 
 /* the selected tangent volume kernels, over the x tiles [tx0, tx1) (tiles of 2 elements)
- * where the kernel takes a range, else over the whole mesh */
+ * where the kernel takes a range, else over the whole mesh; zero: clear the values first */
 template <typename T>
-int launch_tan_volume_x(igab_ctx *c, const igab_geom &g, const double *dU, T *dv, int tx0, int tx1)
+int launch_tan_volume_x(igab_ctx *c, const igab_geom &g, const double *dU, T *dv, int tx0, int tx1, bool zero)
 {
     if (c->phys == IGAB_PHYS_GETIME || (sizeof(T) == 8 ? c->tan_kernel : c->tan32_kernel) == 1)
-        return igab_launch_tan_sf(c, dU, dv, sizeof(T) == 8 ? IGAB_PREC_FP64 : IGAB_PREC_FP32, tx0, tx1);
+        return igab_launch_tan_sf(c, dU, dv, sizeof(T) == 8 ? IGAB_PREC_FP64 : IGAB_PREC_FP32, tx0, tx1, zero);
+    if (zero) {
+        IGAB_CUDA_TRY(cudaMemsetAsync(dv, 0, (size_t)c->nnz * sizeof(T), c->stream));
+        igab_mark(c, 3);
+    }
     return launch_tan_volume<T, 2>(c, g, dU, dv);
 }
 
@@ -889,10 +893,9 @@ template <typename T>
 int launch_tangent_t(igab_ctx *c, const double *dU, T *dv)
 {
     igab_geom g = c->geom();
-    IGAB_CUDA_TRY(cudaMemsetAsync(dv, 0, (size_t)c->nnz * sizeof(T), c->stream));
     igab_mark(c, 3);
     int l0 = c->last_launches;
-    int e = launch_tan_volume_x<T>(c, g, dU, dv, 0, (c->ne[0] + 1) / 2);
+    int e = launch_tan_volume_x<T>(c, g, dU, dv, 0, (c->ne[0] + 1) / 2, true);
     if (e) return e;
     c->nvol_tan = c->last_launches - l0;
     igab_mark(c, 4);
@@ -944,7 +947,7 @@ int launch_tangent_slabs_t(igab_ctx *c, const double *dU, T *dv, long *row_end, 
     for (int i = 0; i <= nb; i++) {
         const int tx0 = i ? b[i - 1] : 0, tx1 = i < nb ? b[i] : ntx;
         const int lv = c->last_launches;
-        int e = launch_tan_volume_x<T>(c, g, dU, dv, tx0, tx1);
+        int e = launch_tan_volume_x<T>(c, g, dU, dv, tx0, tx1, false);
         if (e) return e;
         nvol += c->last_launches - lv;
         if (i == nb) igab_mark(c, 4);

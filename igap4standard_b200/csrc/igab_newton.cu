@@ -140,9 +140,11 @@ int nl_assemble(nl_work &w, int slot, int kind, const double *in, void *out)
     if (!c->nlg) c->nlg = new igab_nl_graphs();
     nl_graph &G = c->nlg->slot[slot];
     if (G.exec && G.in == in && G.out == out && G.kind == kind && G.version == c->sched_version) {
+        int rc = igab_scratch_order(c);
+        if (rc) return rc;
         IGAB_CUDA_TRY(cudaGraphLaunch(G.exec, c->stream));
         w.launches += G.launches;
-        return 0;
+        return igab_scratch_used(c);
     }
     if (G.exec) cudaGraphExecDestroy(G.exec);
     G = nl_graph();
@@ -158,7 +160,9 @@ int nl_assemble(nl_work &w, int slot, int kind, const double *in, void *out)
         cudaGraph_t gr = nullptr;
         cudaError_t e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
+            c->own_capture = true;
             rc = launch_assembly(c, kind, in, out);
+            c->own_capture = false;
             const int n = c->last_launches;
             e = cudaStreamEndCapture(c->stream, &gr);
             if (!rc && e == cudaSuccess) e = cudaGraphInstantiate(&G.exec, gr, 0);

@@ -50,6 +50,12 @@ namespace {
 
 #define SF_THR 256
 #define SF_TE 2
+/* Meshes up to this many elements go through a scratch array of element matrices (143 MB at most) and a gather,
+ * which lets every element run at once; larger ones add tile after tile, colour after colour.  One mesh on one
+ * stream: 8^3 1,079 -> 80 us, 12^3 1,081 -> 213, 16^3 1,096 -> 493, 20^3 1,109 -> 933, 24^3 1,570 -> 1,605
+ * (transient 8^3 1,207 -> 109, 16^3 1,216 -> 695); three meshes on three streams, which fill one another's gaps:
+ * 12^3 369 -> 215 us each, 16^3 476 -> 503, 20^3 648 -> 972. */
+#define SF_ELEM_MAX 4096
 
 /* ---- derivative components m = 0..8: x y z xx xy xz yy yz zz; class = (kx, ky) in the order
  * 0:(0,0) 1:(0,1) 2:(0,2) 3:(1,0) 4:(1,1) 5:(2,0) */
@@ -765,20 +771,59 @@ __device__ __forceinline__ void sf_rows(sf_smem<NR> &S, const igab_geom &g, cons
     (&S.row[0][0])[tid] = R;
 }
 
-/* the element of a tile at or after position le (8: none), le = 4 dx + 2 dy + dz */
-__device__ __forceinline__ int sf_next(const tile_t &T, int le)
-{
-    while (le < 8 && ((le >> 2) >= T.nv[0] || ((le >> 1) & 1) >= T.nv[1] || (le & 1) >= T.nv[2])) le++;
-    return le;
-}
+/* which elements a block does, and where their matrices go: the elements of a 2 x 2 x 2 tile (position
+ * 4 dx + 2 dy + dz ascending) into the CSR values ... */
+template <typename T>
+struct sf_tile_io {
+    tile_t Tl;
+    T *vals;
+    int le;
+    __device__ __forceinline__ bool next(const igab_geom &, sf_elem &E)
+    {
+        do le++;
+        while (le < 8 && ((le >> 2) >= Tl.nv[0] || ((le >> 1) & 1) >= Tl.nv[1] || (le & 1) >= Tl.nv[2]));
+        E = {Tl.e0[0] + (le >> 2), Tl.e0[1] + ((le >> 1) & 1), Tl.e0[2] + (le & 1)};
+        return le < 8;
+    }
+    template <int NR>
+    __device__ __forceinline__ void out(sf_smem<NR> &S, const igab_geom &, const sf_elem &, int k, int s0, int s1, int s2,
+                                        int tid)
+    {
+        sf_scatter<T, NR>(S, vals, k, s0, s1, s2, tid);
+    }
+};
+/* ... or every gridDim-th element of the mesh into a scratch array [element][6 pairs][729] */
+struct sf_elem_io {
+    double *ke;
+    long e, ne;
+    __device__ __forceinline__ bool next(const igab_geom &g, sf_elem &E)
+    {
+        e += gridDim.x;
+        const int i = (int)(e < ne ? e : 0), yz = g.ne[1] * g.ne[2];
+        E = {i / yz, (i % yz) / g.ne[2], i % g.ne[2]};
+        return e < ne;
+    }
+    template <int NR>
+    __device__ __forceinline__ void out(sf_smem<NR> &S, const igab_geom &g, const sf_elem &E, int k, int s0, int s1,
+                                        int s2, int tid)
+    {
+        /* rows 0 bring the pairs (0,0) (0,1) (0,2), rows 1 (1,1) (1,2), rows 2 (2,2): slot s_l, l >= k */
+        double *o = ke + (((long)E.ex * g.ne[1] + E.ey) * g.ne[2] + E.ez) * 4374 + (k == 0 ? 0 : (k == 1 ? 3 : 5)) * 729;
+        for (int l = k; l < 3; l++, o += 729) {
+            const double *K = SF_KSLOT(S, l == 0 ? s0 : (l == 1 ? s1 : s2));
+            for (int i = tid; i < 729; i += SF_THR) o[i] = K[i];
+        }
+    }
+};
 
-template <typename T, int NR>
-__device__ __forceinline__ void sf_tile(const igab_geom &g, const sf_coef &C, const tile_t &Tl,
-                                        const double *__restrict__ U, T *__restrict__ vals, sf_smem<NR> &S)
+template <int NR, class IO>
+__device__ __forceinline__ void sf_run(const igab_geom &g, const sf_coef &C, IO &io, const double *__restrict__ U,
+                                       sf_smem<NR> &S)
 {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    int le = sf_next(Tl, 0), buf = 0;
-    sf_elem E = {Tl.e0[0] + (le >> 2), Tl.e0[1] + ((le >> 1) & 1), Tl.e0[2] + (le & 1)};
+    int buf = 0;
+    sf_elem E;
+    if (!io.next(g, E)) return;
     sf_load<NR>(S, g, U, E, buf, tid);
     sf_copy_wait();
     __syncthreads();
@@ -803,8 +848,8 @@ __device__ __forceinline__ void sf_tile(const igab_geom &g, const sf_coef &C, co
     else sf_s2<NR, 1, DG>(S, tab[1], lane, warp & 3);
 
     while (true) {
-        const int ln = sf_next(Tl, le + 1);
-        const sf_elem En = {Tl.e0[0] + (ln >> 2), Tl.e0[1] + ((ln >> 1) & 1), Tl.e0[2] + (ln & 1)};
+        sf_elem En;
+        const bool more = io.next(g, En);
         const double(*tab)[IGAB_TAB1D] = S.tab[buf];
         /* pairs in the order (0,0) (0,1) (0,2) (1,1) (1,2) (2,2), slots 0 1 2 3 0 4 */
         for (int p = 0; p < 6; p++) {
@@ -821,28 +866,27 @@ __device__ __forceinline__ void sf_tile(const igab_geom &g, const sf_coef &C, co
             if (dg) { SF_S2_(true) } else { SF_S2_(false) }
             if (p == 0) sf_rows<NR>(S, g, E, tid);
             if (p == 3) sf_fix_zy<NR>(S, 0, 1, 2, 3, warp, lane);
-            if (p == 4) sf_scatter<T, NR>(S, vals, 0, 0, 1, 2, tid);
+            if (p == 4) io.out(S, g, E, 0, 0, 1, 2, tid);
             if (p == 5) sf_fix_zy<NR>(S, 3, 0, 0, 2, warp, lane);
             __syncthreads();
         }
-        if (ln < 8) sf_load<NR>(S, g, U, En, buf ^ 1, tid);
+        if (more) sf_load<NR>(S, g, U, En, buf ^ 1, tid);
         sf_s3_all<NR, true>(S, tab[0], SF_KSLOT(S, 4), warp, lane);
         sf_fix_x<NR>(S, 3, 0, 0, 2, tid);
         sf_copy_wait();
         __syncthreads();
         sf_fix_zy<NR>(S, 4, 4, 4, 1, warp, lane);
-        sf_scatter<T, NR>(S, vals, 1, 1, 3, 0, tid);
-        if (ln < 8) sf_interp_z<NR>(S, buf ^ 1, tid);
+        io.out(S, g, E, 1, 1, 3, 0, tid);
+        if (more) sf_interp_z<NR>(S, buf ^ 1, tid);
         __syncthreads();
         sf_fix_x<NR>(S, 4, 4, 4, 1, tid);
-        if (ln < 8) sf_interp_y<NR>(S, buf ^ 1, tid);
+        if (more) sf_interp_y<NR>(S, buf ^ 1, tid);
         __syncthreads();
-        sf_scatter<T, NR>(S, vals, 2, 2, 0, 4, tid);
-        if (ln < 8) sf_interp_x<NR>(S, g, C, buf ^ 1, tid);
+        io.out(S, g, E, 2, 2, 0, 4, tid);
+        if (more) sf_interp_x<NR>(S, g, C, buf ^ 1, tid);
         __syncthreads();
-        if (ln >= 8) break;
+        if (!more) break;
         buf ^= 1;
-        le = ln;
         E = En;
         sf_point_data<NR>(S, g, C, buf, tid);
         __syncthreads();
@@ -859,9 +903,75 @@ __global__ void __launch_bounds__(SF_THR, NR == 1 ? 2 : 1) k_tan_sf(igab_geom g,
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     sf_smem<NR> &S = *reinterpret_cast<sf_smem<NR> *>(smem_raw);
-    tile_t Tl;
-    if (!decode_tile(g, SF_TE, colour, tile0 + blockIdx.x, Tl)) return;
-    sf_tile<T, NR>(g, C, Tl, U, vals, S);
+    sf_tile_io<T> io;
+    if (!decode_tile(g, SF_TE, colour, tile0 + blockIdx.x, io.Tl)) return;
+    io.vals = vals;
+    io.le = -1;
+    sf_run<NR>(g, C, io, U, S);
+}
+
+/* every element matrix of a mesh into a scratch array */
+template <int NR>
+__global__ void __launch_bounds__(SF_THR, NR == 1 ? 2 : 1) k_tan_sf_elem(igab_geom g, sf_coef C,
+                                                                         const double *__restrict__ U,
+                                                                         double *__restrict__ ke, long ne)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    sf_smem<NR> &S = *reinterpret_cast<sf_smem<NR> *>(smem_raw);
+    sf_elem_io io = {ke, (long)blockIdx.x - (long)gridDim.x, ne};
+    sf_run<NR>(g, C, io, U, S);
+}
+
+/* CSR values from the scratch array.  One block per control point, one thread per column (cx, cy, cz, l) of its
+ * rows, the three rows together (one index computation, four loads per element).  An entry receives its at most
+ * 27 element values one by one in the order of the coloured launches (colour position, then position in the
+ * tile) and in the same precision, so the values equal theirs bit for bit. */
+template <typename T>
+__global__ void __launch_bounds__(384) k_tan_gather(igab_geom g, const double *__restrict__ ke, T *__restrict__ vals,
+                                                    int order)
+{
+    const int cp = blockIdx.x, s = threadIdx.x;
+    const int z = cp % g.nb[2], y = (cp / g.nb[2]) % g.nb[1], x = cp / (g.nb[2] * g.nb[1]);
+    const int x0 = max(x - 2, 0), y0 = max(y - 2, 0), y1 = min(y + 2, g.nb[1] - 1);
+    const int z0 = max(z - 2, 0), z1 = min(z + 2, g.nb[2] - 1);
+    const int nyb = y1 - y0 + 1, nzb = z1 - z0 + 1;
+    const int r0 = g.rowptr[3 * cp], len = g.rowptr[3 * cp + 1] - r0;
+    if (s >= len) return;
+    const int l = s % 3, c = s / 3, cz = z0 + c % nzb, cy = y0 + (c / nzb) % nyb, cx = x0 + c / (nzb * nyb);
+    /* per direction the elements that hold both points, by the parity of their tile */
+    const int P[3] = {x, y, z}, Q[3] = {cx, cy, cz};
+    int lo[3][2], hi[3][2];
+#pragma unroll
+    for (int d = 0; d < 3; d++)
+        elem_parity_ranges(max(max(P[d], Q[d]) - 2, 0), min(min(P[d], Q[d]), g.ne[d] - 1) + 1, lo[d], hi[d]);
+    int off[3];   /* pair (min(k,l), max(k,l)) */
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const int u = min(k, l), v = max(k, l);
+        off[k] = 729 * (2 * u - (u >> 1) + v);
+    }
+    T acc[3] = {T(0), T(0), T(0)};
+#pragma unroll 1
+    for (int kp = 0; kp < 8; kp++) {
+        const int col = igab_colour_at(order, kp), px = col >> 2, py = (col >> 1) & 1, pz = col & 1;
+        for (int ex = px ? lo[0][1] : lo[0][0]; ex < (px ? hi[0][1] : hi[0][0]); ex++)
+            for (int ey = py ? lo[1][1] : lo[1][0]; ey < (py ? hi[1][1] : hi[1][0]); ey++)
+                for (int ez = pz ? lo[2][1] : lo[2][0]; ez < (pz ? hi[2][1] : hi[2][0]); ez++) {
+                    const double *K = ke + (((long)ex * g.ne[1] + ey) * g.ne[2] + ez) * 4374;
+                    const int ax = x - ex, ay = y - ey, az = z - ez, bx = cx - ex, by = cy - ey, bz = cz - ez;
+                    const int i = (3 * ax + bx) * 81 + (3 * ay + by) * 9 + 3 * az + bz;
+                    const int it = (3 * bx + ax) * 81 + (3 * by + ay) * 9 + 3 * bz + az;
+                    double v[3];
+#pragma unroll
+                    for (int k = 0; k < 3; k++) v[k] = __ldg(K + off[k] + (k <= l ? i : it));
+                    const double w = __ldg(K + off[l == 0 ? 0 : (l == 1 ? 1 : 2)] + it);
+#pragma unroll
+                    for (int k = 0; k < 3; k++) acc[k] += T(k == l ? v[k] + w : v[k]);
+                }
+    }
+    T *o = vals + r0 + s;
+#pragma unroll
+    for (int k = 0; k < 3; k++) o[(long)k * len] = acc[k];
 }
 
 /* persistent over the tiles of every instance of a batch */
@@ -873,18 +983,44 @@ __global__ void __launch_bounds__(SF_THR, 2) k_tan_sf_batch(igab_batch_dev B, co
     sf_smem<1> &S = *reinterpret_cast<sf_smem<1> *>(smem_raw);
     __shared__ batch_slot sl;
     while (batch_next(B, sl)) {
-        tile_t Tl;
-        decode_tile(sl.g, SF_TE, sl.colour, sl.tile, Tl);
+        sf_tile_io<T> io;
+        decode_tile(sl.g, SF_TE, sl.colour, sl.tile, io.Tl);
+        io.vals = vals + B.nnz_off[sl.inst];
+        io.le = -1;
         const sf_coef C = sf_coef_ge(sl.g);
-        sf_tile<T, 1>(sl.g, C, Tl, U + B.dof_off[sl.inst], vals + B.nnz_off[sl.inst], S);
+        sf_run<1>(sl.g, C, io, U + B.dof_off[sl.inst], S);
         batch_done(B, sl);
     }
 }
 
+int sm_count(int device)
+{
+    int n = 0;
+    return cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && n > 0 ? n : 148;
+}
+
 template <typename T, int NR>
-int launch_sf(igab_ctx *c, const igab_geom &g, const sf_coef &C, const double *dU, T *dv, int tx0, int tx1)
+int launch_sf(igab_ctx *c, const igab_geom &g, const sf_coef &C, const double *dU, T *dv, int tx0, int tx1, bool zero)
 {
     const size_t sm = sizeof(sf_smem<NR>);
+    double *ke = nullptr;
+    if (tx0 == 0 && tx1 == (g.ne[0] + 1) / 2 && c->nel <= SF_ELEM_MAX) {
+        int rc = igab_scratch(c, IGAB_SCRATCH_TAN, (size_t)c->nel * 4374 * sizeof(double), &ke);
+        if (rc) return rc;
+    }
+    if (ke) {
+        IGAB_CUDA_TRY(cudaFuncSetAttribute(k_tan_sf_elem<NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        const long cap = (NR == 1 ? 2L : 1L) * sm_count(c->device);
+        k_tan_sf_elem<NR><<<(unsigned)(c->nel < cap ? c->nel : cap), SF_THR, sm, c->stream>>>(g, C, dU, ke, c->nel);
+        k_tan_gather<T><<<(unsigned)c->ncp, 384, 0, c->stream>>>(g, ke, dv, c->colour_order);
+        c->last_launches += 2;
+        IGAB_CUDA_TRY(cudaGetLastError());
+        return igab_scratch_used(c);
+    }
+    if (zero) {
+        IGAB_CUDA_TRY(cudaMemsetAsync(dv, 0, (size_t)c->nnz * sizeof(T), c->stream));
+        igab_mark(c, 3);
+    }
     IGAB_CUDA_TRY(cudaFuncSetAttribute(k_tan_sf<T, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     for (int k = 0; k < 8; k++) {
         const int colour = igab_colour_at(c->colour_order, k);
@@ -900,16 +1036,17 @@ int launch_sf(igab_ctx *c, const igab_geom &g, const sf_coef &C, const double *d
 
 } /* namespace */
 
-int igab_launch_tan_sf(igab_ctx *c, const double *dU, void *dv, int prec, int tx0, int tx1)
+int igab_launch_tan_sf(igab_ctx *c, const double *dU, void *dv, int prec, int tx0, int tx1, bool zero)
 {
     const igab_geom g = c->geom();
-    if (c->phys == IGAB_PHYS_GETIME) return igab_launch_tan_getime_level(c, dU, dv, prec, 0, tx0, tx1);
+    if (c->phys == IGAB_PHYS_GETIME) return igab_launch_tan_getime_level(c, dU, dv, prec, 0, tx0, tx1, zero);
     const sf_coef C = sf_coef_ge(g);
-    return prec == IGAB_PREC_FP64 ? launch_sf<double, 1>(c, g, C, dU, (double *)dv, tx0, tx1)
-                                  : launch_sf<float, 1>(c, g, C, dU, (float *)dv, tx0, tx1);
+    return prec == IGAB_PREC_FP64 ? launch_sf<double, 1>(c, g, C, dU, (double *)dv, tx0, tx1, zero)
+                                  : launch_sf<float, 1>(c, g, C, dU, (float *)dv, tx0, tx1, zero);
 }
 
-int igab_launch_tan_getime_level(igab_ctx *c, const double *dU, void *dv, int prec, int level, int tx0, int tx1)
+int igab_launch_tan_getime_level(igab_ctx *c, const double *dU, void *dv, int prec, int level, int tx0, int tx1,
+                                 bool zero)
 {
     igab_geom g = c->geom();
     if (level == 1) {          /* d r / d u1 */
@@ -929,8 +1066,8 @@ int igab_launch_tan_getime_level(igab_ctx *c, const double *dU, void *dv, int pr
     C.al = 1.0 / C.r00;
     C.ga = 1.0 / C.r11;
     C.be = -C.r01 * C.al * C.ga;
-    return prec == IGAB_PREC_FP64 ? launch_sf<double, 2>(c, g, C, dU, (double *)dv, tx0, tx1)
-                                  : launch_sf<float, 2>(c, g, C, dU, (float *)dv, tx0, tx1);
+    return prec == IGAB_PREC_FP64 ? launch_sf<double, 2>(c, g, C, dU, (double *)dv, tx0, tx1, zero)
+                                  : launch_sf<float, 2>(c, g, C, dU, (float *)dv, tx0, tx1, zero);
 }
 
 template <typename T>
