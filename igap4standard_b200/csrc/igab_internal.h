@@ -186,7 +186,7 @@ __host__ __device__ inline int igab_colour_at(int order, int k)
 }
 
 /* kernels / launchers (igab_kernels.cu) */
-int igab_launch_residual(igab_ctx *c, const double *dU, double *dR);
+int igab_launch_residual(igab_ctx *c, const double *dU, double *dR, bool scratch = true);   /* scratch: may use igab_scratch */
 int igab_launch_density(igab_ctx *c, const double *dU, double *dHH);   /* igab_density.cu */
 /* igab_krylov.cu: K x on the structured pattern, Jacobi-BiCGStab on the device */
 int igab_launch_spmv(igab_ctx *c, const void *dvals, int prec, const double *dx, double *dy);

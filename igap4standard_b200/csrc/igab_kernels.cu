@@ -32,55 +32,100 @@ namespace {
 
 /* ============================================================ residual */
 
+/* Meshes up to this many elements write element vectors to a scratch array (21 MB at most) that one launch adds up,
+ * instead of eight dependent launches.  One mesh on one stream: 8^3 123 -> 30 us, 16^3 123 -> 60, 24^3 188 -> 137,
+ * 32^3 334 -> 283, 48^3 894 -> 899, 64^3 2025 -> 2113 (transient 8^3 187 -> 34, 32^3 680 -> 643). */
+#define RES_ELEM_MAX 32768
+
 template <int TE, int NL>
 struct res_smem {
     static constexpr int TC = TE + 2;
     static constexpr int NCP = TC * TC * TC;
-    double U[NL][NCP * 3];   /* history levels: t_{n+1}, t_n, t_{n-1} (transient) */
+    double U[NL][NCP * 3];   /* u, or the transient fields (res_stage_fields) */
     double Racc[NCP * 3];
     double tab[3][TE][IGAB_TAB1D];
     double wh[3][TE][IGAB_NQ];
     double xq[3][TE][IGAB_NQ];
-    double A[4][972];
+    double A[4][324];
     double C[4][864];
     double red[4][81];
     double Re[4][81];
 };
 
-/* field and derivatives at this thread's Gauss point from one staged level:
- * z then y contraction in shared memory, x in registers (sum factorisation) */
-template <int TE, int NL>
-__device__ __forceinline__ void res_interp(res_smem<TE, NL> &S, const double *__restrict__ Ul, int group, int gt,
-                                           int lex, int ley, int lez, const double *Bx, const double *By,
-                                           const double *Bz, int qx, int qy, int qz, double u[30])
+/* The transient integrand is a function of the middle m = (u0 + u1) / 2 and the half step h = (u - u0) / 2 of the
+ * segment, and of the inertia / damping force of the values, which is linear in the levels: these three fields
+ * are interpolated, not the levels. */
+__device__ __forceinline__ void res_fields(const igab_geom &g, double u, double u1, double u0, double f[3])
 {
-    constexpr int TC = TE + 2;
-    for (int o = gt; o < 972; o += 64) {
+    f[0] = 0.5 * (u0 + u1);
+    f[1] = 0.5 * (u - u0);
+    f[2] = g.cii * (u - u0) / (2.0 * g.dt) + g.rho * (u + u0 - 2.0 * u1) / (g.dt * g.dt);
+}
+
+/* the derivatives 1..9 of a staged field (TC^3 points, U at the element's first one) at this thread's Gauss point:
+ * z then y contraction in shared memory, x in registers (sum factorisation) */
+template <int TC>
+__device__ __forceinline__ void res_interp(const double *U, double *A, double *C, int group, int gt, const double *Bx,
+                                           const double *By, const double *Bz, int qx, int qy, int qz, double u[30])
+{
+    for (int o = gt; o < 324; o += 64) {
         int i = o % 3, kz = (o / 3) % 3, ay = (o / 9) % 3, ax = (o / 27) % 3, q = o / 81;
-        const double *u0 = &Ul[(((lex + ax) * TC + (ley + ay)) * TC + lez) * 3 + i];
-        S.A[group][o] = Bz[q * 9 + 0 * 3 + kz] * u0[0] + Bz[q * 9 + 1 * 3 + kz] * u0[3] + Bz[q * 9 + 2 * 3 + kz] * u0[6];
+        const double *u0 = U + ((ax * TC + ay) * TC) * 3 + i;
+        A[o] = Bz[q * 9 + 0 * 3 + kz] * u0[0] + Bz[q * 9 + 1 * 3 + kz] * u0[3] + Bz[q * 9 + 2 * 3 + kz] * u0[6];
     }
     group_sync(group);
     for (int o = gt; o < 864; o += 64) {
         int i = o % 3, kk = (o / 3) % 6, ax = (o / 18) % 3, qq = o / 54;
         int qyy = qq & 3, qzz = qq >> 2;
         int ky = kk_ky(kk), kz = kk_kz(kk);
-        const double *a0 = &S.A[group][((qzz * 3 + ax) * 3) * 9 + kz * 3 + i];
-        S.C[group][o] = By[qyy * 9 + 0 * 3 + ky] * a0[0] + By[qyy * 9 + 1 * 3 + ky] * a0[9] + By[qyy * 9 + 2 * 3 + ky] * a0[18];
+        const double *a0 = A + ((qzz * 3 + ax) * 3) * 9 + kz * 3 + i;
+        C[o] = By[qyy * 9 + 0 * 3 + ky] * a0[0] + By[qyy * 9 + 1 * 3 + ky] * a0[9] + By[qyy * 9 + 2 * 3 + ky] * a0[18];
     }
     group_sync(group);
-    const int qq = qy + 4 * qz;
+    const double *c = C + (qy + 4 * qz) * 54;
+    double b[3][3];
 #pragma unroll
-    for (int a = 0; a < 10; a++) {
+    for (int ax = 0; ax < 3; ax++)
 #pragma unroll
-        for (int i = 0; i < 3; i++) {
+        for (int k = 0; k < 3; k++) b[ax][k] = Bx[qx * 9 + ax * 3 + k];
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        u[10 * i] = 0.0;
+#pragma unroll
+        for (int a = 1; a < 10; a++) {
             double s = 0.0;
 #pragma unroll
-            for (int ax = 0; ax < 3; ax++) s += Bx[qx * 9 + ax * 3 + a_kx(a)] * S.C[group][((qq * 3 + ax) * 6 + a_kk(a)) * 3 + i];
+            for (int ax = 0; ax < 3; ax++) s += b[ax][a_kx(a)] * c[(ax * 6 + a_kk(a)) * 3 + i];
             u[10 * i + a] = s;
         }
     }
-    group_sync(group);   /* A and C are reused by the next level */
+    group_sync(group);   /* A and C are reused */
+}
+
+/* the values only */
+template <int TC>
+__device__ __forceinline__ void res_interp_value(const double *U, double *A, double *C, int group, int gt,
+                                                 const double *Bx, const double *By, const double *Bz, int qx, int qy,
+                                                 int qz, double v[3])
+{
+    for (int o = gt; o < 108; o += 64) {
+        int i = o % 3, a = (o / 3) % 9, q = o / 27;
+        const double *u0 = U + ((a / 3) * TC + a % 3) * TC * 3 + i;
+        A[o] = Bz[q * 9] * u0[0] + Bz[q * 9 + 3] * u0[3] + Bz[q * 9 + 6] * u0[6];
+    }
+    group_sync(group);
+    for (int o = gt; o < 144; o += 64) {
+        int i = o % 3, ax = (o / 3) % 3, qq = o / 9, qyy = qq & 3, qzz = qq >> 2;
+        const double *a0 = A + qzz * 27 + ax * 9 + i;
+        C[o] = By[qyy * 9] * a0[0] + By[qyy * 9 + 3] * a0[3] + By[qyy * 9 + 6] * a0[6];
+    }
+    group_sync(group);
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const double *c = C + (qy + 4 * qz) * 9 + i;
+        v[i] = Bx[qx * 9] * c[0] + Bx[qx * 9 + 3] * c[3] + Bx[qx * 9 + 6] * c[6];
+    }
+    group_sync(group);
 }
 
 __device__ __forceinline__ void add_periodic(const igab_geom &g, const double X[3], double u[30])
@@ -93,14 +138,131 @@ __device__ __forceinline__ void add_periodic(const igab_geom &g, const double X[
     }
 }
 
-/* VJP = false: add the tile's element residuals into R.
- * VJP = true: adjoint mode; nothing is added to R, instead grad[e] = lam_e . R_e
- * for every element of the tile (lam with Dirichlet rows already zeroed), i.e.
- * the vector-Jacobian product lam^T dR/dg_e of the scaled residual. */
-template <int TE, bool GT, bool VJP>
+/* The element vector Re[81] of one element by 64 threads (one per Gauss point).  U0..U2: the staged field (u), or
+ * the three transient fields, at the element's first control point in arrays of TC^3 points; A, C, red: scratch of
+ * the group. */
+template <int TC, bool GT>
+__device__ __forceinline__ void res_element(const igab_geom &g, const double *U0, const double *U1, const double *U2,
+                                            double *A, double *C, double *red, double *Re, int group, int gt,
+                                            const double *Bx, const double *By, const double *Bz, const double *xx,
+                                            const double *xy, const double *xz, double w)
+{
+    const int qx = gt & 3, qy = (gt >> 2) & 3, qz = gt >> 4;
+    double r[30];
+    {
+        double u[30];
+        res_interp<TC>(U0, A, C, group, gt, Bx, By, Bz, qx, qy, qz, u);
+        if (g.periodic) {
+            const double X[3] = {xx[qx], xy[qy], xz[qz]};
+            add_periodic(g, X, u);
+        }
+        if (GT) {
+            double h[30], v[3];
+            res_interp<TC>(U1, A, C, group, gt, Bx, By, Bz, qx, qy, qz, h);
+            res_interp_value<TC>(U2, A, C, group, gt, Bx, By, Bz, qx, qy, qz, v);
+            igab_getime_gradient(u, h, g.coef, r);
+#pragma unroll
+            for (int i = 0; i < 3; i++) r[10 * i] = v[i];
+        } else {
+            igab_ge_point<double> P;
+            igab_ge_eval(u, g.coef, P);
+            igab_ge_residual(P, r);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 30; k++) r[k] *= w;
+
+    /* backward step 1: partial sums over x for this point, P1[ax][kk][i] */
+    double P1[3][18];
+#pragma unroll
+    for (int ax = 0; ax < 3; ax++)
+#pragma unroll
+        for (int s = 0; s < 18; s++) P1[ax][s] = 0.0;
+#pragma unroll
+    for (int a = GT ? 0 : 1; a < 10; a++)
+#pragma unroll
+        for (int ax = 0; ax < 3; ax++) {
+            double b = Bx[qx * 9 + ax * 3 + a_kx(a)];
+#pragma unroll
+            for (int i = 0; i < 3; i++) P1[ax][a_kk(a) * 3 + i] += b * r[10 * i + a];
+        }
+    /* reduce-scatter over the 4 x-lanes: lane qx keeps ax = qx (qx < 3) */
+    const int b1 = (qx >> 1) & 1, b0 = qx & 1;
+#pragma unroll
+    for (int s = 0; s < 18; s++) {
+        double x1 = b1 ? P1[0][s] : P1[2][s];
+        double y1 = shfl_xor(x1, 2);
+        double x2 = b1 ? P1[1][s] : 0.0;
+        double y2 = shfl_xor(x2, 2);
+        if (b1) P1[2][s] += y1; else { P1[0][s] += y1; P1[1][s] += y2; }
+    }
+    double Y[18];
+#pragma unroll
+    for (int s = 0; s < 18; s++) {
+        double x = b1 ? P1[2][s] : (b0 ? P1[0][s] : P1[1][s]);
+        double y = shfl_xor(x, 1);
+        double mine = b1 ? P1[2][s] : (b0 ? P1[1][s] : P1[0][s]);
+        Y[s] = mine + y;
+    }
+    /* backward step 2: contract y for ax = qx; P2[ay][kz][i] */
+    double P2[3][9];
+#pragma unroll
+    for (int ay = 0; ay < 3; ay++)
+#pragma unroll
+        for (int s = 0; s < 9; s++) P2[ay][s] = 0.0;
+#pragma unroll
+    for (int kk = 0; kk < 6; kk++)
+#pragma unroll
+        for (int ay = 0; ay < 3; ay++) {
+            double b = By[qy * 9 + ay * 3 + kk_ky(kk)];
+#pragma unroll
+            for (int i = 0; i < 3; i++) P2[ay][kk_kz(kk) * 3 + i] += b * Y[kk * 3 + i];
+        }
+    /* reduce-scatter over the 4 y-lanes (lane bits 2,3): lane qy keeps ay = qy */
+    const int c1 = (qy >> 1) & 1, c0 = qy & 1;
+#pragma unroll
+    for (int s = 0; s < 9; s++) {
+        double x1 = c1 ? P2[0][s] : P2[2][s];
+        double y1 = shfl_xor(x1, 8);
+        double x2 = c1 ? P2[1][s] : 0.0;
+        double y2 = shfl_xor(x2, 8);
+        if (c1) P2[2][s] += y1; else { P2[0][s] += y1; P2[1][s] += y2; }
+    }
+    double Z[9];
+#pragma unroll
+    for (int s = 0; s < 9; s++) {
+        double x = c1 ? P2[2][s] : (c0 ? P2[0][s] : P2[1][s]);
+        double y = shfl_xor(x, 4);
+        double mine = c1 ? P2[2][s] : (c0 ? P2[1][s] : P2[0][s]);
+        Z[s] = mine + y;
+    }
+    /* backward step 3: contract z for (ax, ay) = (qx, qy); sum over qz */
+    double P3[9];
+#pragma unroll
+    for (int az = 0; az < 3; az++)
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            double s = 0.0;
+#pragma unroll
+            for (int kz = 0; kz < 3; kz++) s += Bz[qz * 9 + az * 3 + kz] * Z[kz * 3 + i];
+            P3[az * 3 + i] = s;
+        }
+#pragma unroll
+    for (int s = 0; s < 9; s++) P3[s] += shfl_xor(P3[s], 16);
+    const bool owner = qx < 3 && qy < 3 && (qz & 1) == 0;
+    if (owner && qz == 2)
+#pragma unroll
+        for (int s = 0; s < 9; s++) red[(qx * 3 + qy) * 9 + s] = P3[s];
+    group_sync(group);
+    if (owner && qz == 0)
+#pragma unroll
+        for (int s = 0; s < 9; s++) Re[(qx * 3 + qy) * 9 + s] = P3[s] + red[(qx * 3 + qy) * 9 + s];
+}
+
+/* add the tile's element residuals into R */
+template <int TE, bool GT>
 __device__ __forceinline__ void res_tile(const igab_geom &g, const tile_t &T, const double *__restrict__ U,
-                                         double *__restrict__ R, const double *__restrict__ lam,
-                                         double *__restrict__ grad, res_smem<TE, GT ? 3 : 1> &S)
+                                         double *__restrict__ R, res_smem<TE, GT ? 3 : 1> &S)
 {
     constexpr int NL = GT ? 3 : 1;
     constexpr int TC = TE + 2;
@@ -114,12 +276,14 @@ __device__ __forceinline__ void res_tile(const igab_geom &g, const tile_t &T, co
         int lz = cp % TC, ly = (cp / TC) % TC, lx = cp / (TC * TC);
         const bool in = lx < T.nv[0] + 2 && ly < T.nv[1] + 2 && lz < T.nv[2] + 2;
         const long gi = in ? 3 * cp_index(g, T.e0[0] + lx, T.e0[1] + ly, T.e0[2] + lz) + i : 0;
+        if constexpr (GT) {
+            double f[3] = {0.0, 0.0, 0.0};
+            if (in) res_fields(g, U[gi], g.hist1[gi], g.hist0[gi], f);
 #pragma unroll
-        for (int l = 0; l < NL; l++) {
-            const double *src = l == 0 ? U : (l == 1 ? g.hist1 : g.hist0);
-            S.U[l][idx] = in ? src[gi] : 0.0;
-        }
-        S.Racc[idx] = VJP ? (in ? lam[gi] : 0.0) : 0.0;   /* adjoint mode keeps lam here */
+            for (int l = 0; l < NL; l++) S.U[l][idx] = f[l];
+        } else
+            S.U[0][idx] = in ? U[gi] : 0.0;
+        S.Racc[idx] = 0.0;
     }
     for (int idx = tid; idx < 3 * TE * IGAB_TAB1D; idx += blockDim.x) {
         int d = idx / (TE * IGAB_TAB1D), r = idx % (TE * IGAB_TAB1D), le = r / IGAB_TAB1D, o = r % IGAB_TAB1D;
@@ -135,149 +299,21 @@ __device__ __forceinline__ void res_tile(const igab_geom &g, const tile_t &T, co
 
     const int group = tid >> 6;
     const int gt = tid & 63;
-    const int qx = gt & 3, qy = (gt >> 2) & 3, qz = gt >> 4;
 
     for (int base = 0; base < NEL; base += 4) {
         const int le = base + group;
         const int lex = le / (TE * TE), ley = (le / TE) % TE, lez = le % TE;
         const bool valid = lex < T.nv[0] && ley < T.nv[1] && lez < T.nv[2];
         if (valid) {
-            const double *Bx = S.tab[0][lex];
-            const double *By = S.tab[1][ley];
-            const double *Bz = S.tab[2][lez];
-            double u[30];
-            const double X[3] = {S.xq[0][lex][qx], S.xq[1][ley][qy], S.xq[2][lez][qz]};
-            res_interp<TE, NL>(S, S.U[0], group, gt, lex, ley, lez, Bx, By, Bz, qx, qy, qz, u);
-            if (g.periodic) add_periodic(g, X, u);
-            /* integrand */
-            double r[30];
-            if (GT) {
-                double u1[30], u0[30];
-                res_interp<TE, NL>(S, S.U[NL > 1 ? 1 : 0], group, gt, lex, ley, lez, Bx, By, Bz, qx, qy, qz, u1);
-                res_interp<TE, NL>(S, S.U[NL > 2 ? 2 : 0], group, gt, lex, ley, lez, Bx, By, Bz, qx, qy, qz, u0);
-                if (g.periodic) {
-                    add_periodic(g, X, u1);
-                    add_periodic(g, X, u0);
-                }
-                igab_getime_residual(u, u1, u0, g.coef, g.rho, g.cii, g.dt, r);
-            } else {
-                igab_ge_point<double> P;
-                igab_ge_eval(u, g.coef, P);
-                igab_ge_residual(P, r);
-            }
+            const int o = ((lex * TC + ley) * TC + lez) * 3;
+            const int qx = gt & 3, qy = (gt >> 2) & 3, qz = gt >> 4;
             const double w = S.wh[0][lex][qx] * S.wh[1][ley][qy] * S.wh[2][lez][qz] *
                              elem_scale(g, T.e0[0] + lex, T.e0[1] + ley, T.e0[2] + lez);
-#pragma unroll
-            for (int k = 0; k < 30; k++) r[k] *= w;
-
-            /* backward step 1: partial sums over x for this point, P1[ax][kk][i] */
-            double P1[3][18];
-#pragma unroll
-            for (int ax = 0; ax < 3; ax++)
-#pragma unroll
-                for (int s = 0; s < 18; s++) P1[ax][s] = 0.0;
-#pragma unroll
-            for (int a = 0; a < 10; a++)
-#pragma unroll
-                for (int ax = 0; ax < 3; ax++) {
-                    double b = Bx[qx * 9 + ax * 3 + a_kx(a)];
-#pragma unroll
-                    for (int i = 0; i < 3; i++) P1[ax][a_kk(a) * 3 + i] += b * r[10 * i + a];
-                }
-            /* reduce-scatter over the 4 x-lanes: lane qx keeps ax = qx (qx < 3) */
-            const int b1 = (qx >> 1) & 1, b0 = qx & 1;
-#pragma unroll
-            for (int s = 0; s < 18; s++) {
-                double x1 = b1 ? P1[0][s] : P1[2][s];
-                double y1 = shfl_xor(x1, 2);
-                double x2 = b1 ? P1[1][s] : 0.0;
-                double y2 = shfl_xor(x2, 2);
-                if (b1) P1[2][s] += y1; else { P1[0][s] += y1; P1[1][s] += y2; }
-            }
-            double Y[18];
-#pragma unroll
-            for (int s = 0; s < 18; s++) {
-                double x = b1 ? P1[2][s] : (b0 ? P1[0][s] : P1[1][s]);
-                double y = shfl_xor(x, 1);
-                double mine = b1 ? P1[2][s] : (b0 ? P1[1][s] : P1[0][s]);
-                Y[s] = mine + y;
-            }
-            /* backward step 2: contract y for ax = qx; P2[ay][kz][i] */
-            double P2[3][9];
-#pragma unroll
-            for (int ay = 0; ay < 3; ay++)
-#pragma unroll
-                for (int s = 0; s < 9; s++) P2[ay][s] = 0.0;
-#pragma unroll
-            for (int kk = 0; kk < 6; kk++)
-#pragma unroll
-                for (int ay = 0; ay < 3; ay++) {
-                    double b = By[qy * 9 + ay * 3 + kk_ky(kk)];
-#pragma unroll
-                    for (int i = 0; i < 3; i++) P2[ay][kk_kz(kk) * 3 + i] += b * Y[kk * 3 + i];
-                }
-            /* reduce-scatter over the 4 y-lanes (lane bits 2,3): lane qy keeps ay = qy */
-            const int c1 = (qy >> 1) & 1, c0 = qy & 1;
-#pragma unroll
-            for (int s = 0; s < 9; s++) {
-                double x1 = c1 ? P2[0][s] : P2[2][s];
-                double y1 = shfl_xor(x1, 8);
-                double x2 = c1 ? P2[1][s] : 0.0;
-                double y2 = shfl_xor(x2, 8);
-                if (c1) P2[2][s] += y1; else { P2[0][s] += y1; P2[1][s] += y2; }
-            }
-            double Z[9];
-#pragma unroll
-            for (int s = 0; s < 9; s++) {
-                double x = c1 ? P2[2][s] : (c0 ? P2[0][s] : P2[1][s]);
-                double y = shfl_xor(x, 4);
-                double mine = c1 ? P2[2][s] : (c0 ? P2[1][s] : P2[0][s]);
-                Z[s] = mine + y;
-            }
-            /* backward step 3: contract z for (ax, ay) = (qx, qy); sum over qz */
-            double P3[9];
-#pragma unroll
-            for (int az = 0; az < 3; az++)
-#pragma unroll
-                for (int i = 0; i < 3; i++) {
-                    double s = 0.0;
-#pragma unroll
-                    for (int kz = 0; kz < 3; kz++) s += Bz[qz * 9 + az * 3 + kz] * Z[kz * 3 + i];
-                    P3[az * 3 + i] = s;
-                }
-#pragma unroll
-            for (int s = 0; s < 9; s++) P3[s] += shfl_xor(P3[s], 16);
-            const bool owner = qx < 3 && qy < 3 && (qz & 1) == 0;
-            if (owner && qz == 2)
-#pragma unroll
-                for (int s = 0; s < 9; s++) S.red[group][(qx * 3 + qy) * 9 + s] = P3[s];
-            group_sync(group);
-            if (owner && qz == 0)
-#pragma unroll
-                for (int s = 0; s < 9; s++) S.Re[group][(qx * 3 + qy) * 9 + s] = P3[s] + S.red[group][(qx * 3 + qy) * 9 + s];
+            res_element<TC, GT>(g, S.U[0] + o, S.U[NL > 1 ? 1 : 0] + o, S.U[NL > 2 ? 2 : 0] + o, S.A[group], S.C[group],
+                                S.red[group], S.Re[group], group, gt, S.tab[0][lex], S.tab[1][ley], S.tab[2][lez],
+                                S.xq[0][lex], S.xq[1][ley], S.xq[2][lez], w);
         }
         __syncthreads();
-        if (VJP) {
-            /* one warp per element: grad_e = sum_k Re[k] lam[k], fixed order */
-            const int w = tid >> 5, lane = tid & 31;
-            if (w < 4) {
-                const int e = base + w;
-                const int ex = e / (TE * TE), ey = (e / TE) % TE, ez = e % TE;
-                if (e < NEL && ex < T.nv[0] && ey < T.nv[1] && ez < T.nv[2]) {
-                    double s = 0.0;
-                    for (int k = lane; k < 81; k += 32) {
-                        const int i = k % 3, az = (k / 3) % 3, ay = (k / 9) % 3, ax = k / 27;
-                        s += S.Re[w][k] * S.Racc[(((ex + ax) * TC + (ey + ay)) * TC + (ez + az)) * 3 + i];
-                    }
-#pragma unroll
-                    for (int m = 16; m >= 1; m >>= 1) s += shfl_xor(s, m);
-                    if (lane == 0)
-                        grad[((long)(T.e0[0] + ex) * g.ne[1] + (T.e0[1] + ey)) * g.ne[2] + (T.e0[2] + ez)] = s;
-                }
-            }
-            __syncthreads();
-            continue;
-        }
         /* ---- fixed-order accumulation of the (up to) 4 element vectors into the tile */
         for (int idx = tid; idx < NCP * 3; idx += blockDim.x) {
             int i = idx % 3, cp = idx / 3;
@@ -296,7 +332,6 @@ __device__ __forceinline__ void res_tile(const igab_geom &g, const tile_t &T, co
         }
         __syncthreads();
     }
-    if (VJP) return;
     /* ---- add the tile into the global residual (no other tile of this colour touches these points) */
     for (int idx = tid; idx < NCP * 3; idx += blockDim.x) {
         int i = idx % 3, cp = idx / 3;
@@ -308,16 +343,109 @@ __device__ __forceinline__ void res_tile(const igab_geom &g, const tile_t &T, co
     }
 }
 
-template <int TE, bool GT, bool VJP>
-__global__ void __launch_bounds__(256) k_res_volume(igab_geom g, const double *__restrict__ U,
-                                                    double *__restrict__ R, int colour,
-                                                    const double *__restrict__ lam, double *__restrict__ grad)
+template <int TE, bool GT>
+__global__ void __launch_bounds__(256, GT ? 1 : 2) k_res_volume(igab_geom g, const double *__restrict__ U,
+                                                    double *__restrict__ R, int colour)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     res_smem<TE, GT ? 3 : 1> &S = *reinterpret_cast<res_smem<TE, GT ? 3 : 1> *>(smem_raw);
     tile_t T;
     if (!decode_tile(g, TE, colour, blockIdx.x, T)) return;
-    res_tile<TE, GT, VJP>(g, T, U, R, lam, grad, S);
+    res_tile<TE, GT>(g, T, U, R, S);
+}
+
+/* Four elements per block, 64 threads each, without any dependence between elements: the element vectors
+ * [element][81] (VJP = false; k_res_gather adds them up), or grad[e] = lam_e . R_e (VJP = true). */
+template <bool GT>
+struct res_elem_smem {
+    double U[4][GT ? 3 : 1][81];
+    double lam[4][81];
+    double tab[4][3][IGAB_TAB1D];
+    double wh[4][3][IGAB_NQ];
+    double xq[4][3][IGAB_NQ];
+    double A[4][324];
+    double C[4][864];
+    double red[4][81];
+    double Re[4][81];
+};
+template <bool GT, bool VJP>
+__global__ void __launch_bounds__(256, GT ? 1 : 2) k_res_elem(igab_geom g, const double *__restrict__ U, double *__restrict__ out,
+                                                  const double *__restrict__ lam, long ne)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    res_elem_smem<GT> &S = *reinterpret_cast<res_elem_smem<GT> *>(smem_raw);
+    const int group = threadIdx.x >> 6, gt = threadIdx.x & 63;
+    const long e = 4L * blockIdx.x + group;
+    if (e >= ne) return;
+    const int yz = g.ne[1] * g.ne[2], ex = (int)(e / yz), ey = (int)(e % yz) / g.ne[2], ez = (int)(e % yz) % g.ne[2];
+    for (int o = gt; o < 81; o += 64) {
+        const int a = o / 3;
+        const long gi = 3 * cp_index(g, ex + a / 9, ey + (a / 3) % 3, ez + a % 3) + o % 3;
+        if constexpr (GT) {
+            double f[3];
+            res_fields(g, U[gi], g.hist1[gi], g.hist0[gi], f);
+#pragma unroll
+            for (int l = 0; l < 3; l++) S.U[group][l][o] = f[l];
+        } else
+            S.U[group][0][o] = U[gi];
+        if (VJP) S.lam[group][o] = lam[gi];
+    }
+    for (int o = gt; o < 3 * IGAB_TAB1D; o += 64) {
+        const int d = o / IGAB_TAB1D, i = o % IGAB_TAB1D, ed = d == 0 ? ex : (d == 1 ? ey : ez);
+        S.tab[group][d][i] = g.tab[d][(long)ed * IGAB_TAB1D + i];
+    }
+    if (gt < 12) {
+        const int d = gt >> 2, ed = d == 0 ? ex : (d == 1 ? ey : ez);
+        S.wh[group][d][gt & 3] = g.wh[d][(long)ed * IGAB_NQ + (gt & 3)];
+        S.xq[group][d][gt & 3] = g.xq[d][(long)ed * IGAB_NQ + (gt & 3)];
+    }
+    group_sync(group);
+    const int qx = gt & 3, qy = (gt >> 2) & 3, qz = gt >> 4;
+    const double w = S.wh[group][0][qx] * S.wh[group][1][qy] * S.wh[group][2][qz] * elem_scale(g, ex, ey, ez);
+    res_element<3, GT>(g, S.U[group][0], S.U[group][GT ? 1 : 0], S.U[group][GT ? 2 : 0], S.A[group], S.C[group],
+                       S.red[group], S.Re[group], group, gt, S.tab[group][0], S.tab[group][1], S.tab[group][2],
+                       S.xq[group][0], S.xq[group][1], S.xq[group][2], w);
+    group_sync(group);
+    if (!VJP) {
+        for (int o = gt; o < 81; o += 64) out[e * 81 + o] = S.Re[group][o];
+    } else if (gt < 32) {
+        double s = 0.0;
+        for (int k = gt; k < 81; k += 32) s += S.Re[group][k] * S.lam[group][k];
+#pragma unroll
+        for (int m = 16; m >= 1; m >>= 1) s += shfl_xor(s, m);
+        if (gt == 0) out[e] = s;
+    }
+}
+
+/* R from the element vectors, one thread per dof.  The at most 27 contributions are added as the coloured
+ * launches add them (per colour the tile's elements first, in tile order, then the tile's sum), so R equals
+ * theirs bit for bit. */
+__global__ void __launch_bounds__(256) k_res_gather(igab_geom g, const double *__restrict__ re, double *__restrict__ R,
+                                                 int order)
+{
+    const long r = blockIdx.x * 256L + threadIdx.x;
+    if (r >= g.ndof) return;
+    const int cp = (int)(r / 3), i = (int)(r % 3);
+    const int P[3] = {cp / (g.nb[2] * g.nb[1]), (cp / g.nb[2]) % g.nb[1], cp % g.nb[2]};
+    int lo[3][2], hi[3][2];
+#pragma unroll
+    for (int d = 0; d < 3; d++) elem_parity_ranges(max(P[d] - 2, 0), min(P[d], g.ne[d] - 1) + 1, lo[d], hi[d]);
+    double acc = 0.0;
+#pragma unroll 1
+    for (int kp = 0; kp < 8; kp++) {
+        const int col = igab_colour_at(order, kp), px = col >> 2, py = (col >> 1) & 1, pz = col & 1;
+        double t = 0.0;
+        bool any = false;
+        for (int ex = px ? lo[0][1] : lo[0][0]; ex < (px ? hi[0][1] : hi[0][0]); ex++)
+            for (int ey = py ? lo[1][1] : lo[1][0]; ey < (py ? hi[1][1] : hi[1][0]); ey++)
+                for (int ez = pz ? lo[2][1] : lo[2][0]; ez < (pz ? hi[2][1] : hi[2][0]); ez++) {
+                    const long e = ((long)ex * g.ne[1] + ey) * g.ne[2] + ez;
+                    t += __ldg(re + e * 81 + ((P[0] - ex) * 9 + (P[1] - ey) * 3 + (P[2] - ez)) * 3 + i);
+                    any = true;
+                }
+        if (any) acc += t;
+    }
+    R[r] = acc;
 }
 
 /* Neumann surface terms (src/snesiga_Residual.c:243-320): one thread per
@@ -727,7 +855,7 @@ __global__ void __launch_bounds__(256, 2) k_res_batch(igab_batch_dev B, const do
         tile_t T;
         decode_tile(sl.g, 2, sl.colour, sl.tile, T);
         const long off = B.dof_off[sl.inst];
-        res_tile<2, false, false>(sl.g, T, U + off, R + off, nullptr, nullptr, S);
+        res_tile<2, false>(sl.g, T, U + off, R + off, S);
         batch_done(B, sl);
     }
 }
@@ -831,17 +959,16 @@ __global__ void k_check_finite(const T *__restrict__ v, long n, int *__restrict_
     if (__syncthreads_or(bad) && threadIdx.x == 0) atomicExch(flag, 1);
 }
 
-template <int TE, bool GT, bool VJP = false>
-int launch_res_volume_t(igab_ctx *c, const igab_geom &g, const double *dU, double *dR,
-                        const double *dlam = nullptr, double *dgrad = nullptr)
+template <int TE, bool GT>
+int launch_res_volume_t(igab_ctx *c, const igab_geom &g, const double *dU, double *dR)
 {
     size_t sm = sizeof(res_smem<TE, GT ? 3 : 1>);
-    IGAB_CUDA_TRY(cudaFuncSetAttribute(k_res_volume<TE, GT, VJP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    IGAB_CUDA_TRY(cudaFuncSetAttribute(k_res_volume<TE, GT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     for (int k = 0; k < 8; k++) {
         const int colour = igab_colour_at(c->colour_order, k);
         long nblk = tiles_of_colour(g, TE, colour);
         if (nblk == 0) continue;
-        k_res_volume<TE, GT, VJP><<<(unsigned)nblk, 256, sm, c->stream>>>(g, dU, dR, colour, dlam, dgrad);
+        k_res_volume<TE, GT><<<(unsigned)nblk, 256, sm, c->stream>>>(g, dU, dR, colour);
         c->last_launches++;
     }
     IGAB_CUDA_TRY(cudaGetLastError());
@@ -967,18 +1094,43 @@ int launch_tangent_slabs_t(igab_ctx *c, const double *dU, T *dv, long *row_end, 
 
 } /* namespace */
 
-int igab_launch_residual(igab_ctx *c, const double *dU, double *dR)
+/* element vectors to scratch, then the gather (*done = false: no scratch, use the coloured launches) */
+template <bool GT>
+static int launch_res_elem(igab_ctx *c, const igab_geom &g, const double *dU, double *dR, bool *done)
+{
+    *done = false;
+    if (c->tile_res != 2 || c->nel > RES_ELEM_MAX) return 0;
+    double *re = nullptr;
+    int rc = igab_scratch(c, IGAB_SCRATCH_RES, (size_t)c->nel * 81 * sizeof(double), &re);
+    if (rc || !re) return rc;
+    const size_t sm = sizeof(res_elem_smem<GT>);
+    IGAB_CUDA_TRY(cudaFuncSetAttribute(k_res_elem<GT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    k_res_elem<GT, false><<<(unsigned)((c->nel + 3) / 4), 256, sm, c->stream>>>(g, dU, re, nullptr, c->nel);
+    k_res_gather<<<(unsigned)((c->ndof + 255) / 256), 256, 0, c->stream>>>(g, re, dR, c->colour_order);
+    c->last_launches += 2;
+    IGAB_CUDA_TRY(cudaGetLastError());
+    *done = true;
+    return igab_scratch_used(c);
+}
+
+int igab_launch_residual(igab_ctx *c, const double *dU, double *dR, bool scratch)
 {
     c->last_launches = 0;
     igab_geom g = c->geom();
-    IGAB_CUDA_TRY(cudaMemsetAsync(dR, 0, (size_t)c->ndof * sizeof(double), c->stream));
     igab_mark(c, 0);
-    int e;
-    if (c->phys == IGAB_PHYS_GETIME)
-        e = c->tile_res == 4 ? launch_res_volume_t<4, true>(c, g, dU, dR) : launch_res_volume_t<2, true>(c, g, dU, dR);
-    else
-        e = c->tile_res == 4 ? launch_res_volume_t<4, false>(c, g, dU, dR) : launch_res_volume_t<2, false>(c, g, dU, dR);
+    bool done = false;
+    int e = !scratch ? 0 : (c->phys == IGAB_PHYS_GETIME ? launch_res_elem<true>(c, g, dU, dR, &done)
+                                                        : launch_res_elem<false>(c, g, dU, dR, &done));
     if (e) return e;
+    if (!done) {
+        IGAB_CUDA_TRY(cudaMemsetAsync(dR, 0, (size_t)c->ndof * sizeof(double), c->stream));
+        igab_mark(c, 0);
+        if (c->phys == IGAB_PHYS_GETIME)
+            e = c->tile_res == 4 ? launch_res_volume_t<4, true>(c, g, dU, dR) : launch_res_volume_t<2, true>(c, g, dU, dR);
+        else
+            e = c->tile_res == 4 ? launch_res_volume_t<4, false>(c, g, dU, dR) : launch_res_volume_t<2, false>(c, g, dU, dR);
+        if (e) return e;
+    }
     c->nvol_res = c->last_launches;
     igab_mark(c, 1);
     if ((c->neumann_nonzero || c->force_neumann) && c->n_neu_rows > 0) {
@@ -1021,6 +1173,17 @@ int igab_launch_exp_scale(igab_ctx *c, const double *dg)
     return 0;
 }
 
+template <bool GT>
+static int launch_res_vjp(igab_ctx *c, const igab_geom &g, const double *dU, double *dgrad)
+{
+    const size_t sm = sizeof(res_elem_smem<GT>);
+    IGAB_CUDA_TRY(cudaFuncSetAttribute(k_res_elem<GT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    k_res_elem<GT, true><<<(unsigned)((c->nel + 3) / 4), 256, sm, c->stream>>>(g, dU, dgrad, c->d_lam, c->nel);
+    c->last_launches++;
+    IGAB_CUDA_TRY(cudaGetLastError());
+    return 0;
+}
+
 /* grad_e = lam~^T dR/dg_e with lam~ = lam outside the Dirichlet rows (c->d_lam is scratch) */
 int igab_launch_adjoint_dRdg(igab_ctx *c, const double *dU, const double *dlam, double *dgrad)
 {
@@ -1031,11 +1194,7 @@ int igab_launch_adjoint_dRdg(igab_ctx *c, const double *dU, const double *dlam, 
         c->last_launches++;
         IGAB_CUDA_TRY(cudaGetLastError());
     }
-    if (c->phys == IGAB_PHYS_GETIME)
-        return c->tile_res == 4 ? launch_res_volume_t<4, true, true>(c, g, dU, nullptr, c->d_lam, dgrad)
-                                : launch_res_volume_t<2, true, true>(c, g, dU, nullptr, c->d_lam, dgrad);
-    return c->tile_res == 4 ? launch_res_volume_t<4, false, true>(c, g, dU, nullptr, c->d_lam, dgrad)
-                            : launch_res_volume_t<2, false, true>(c, g, dU, nullptr, c->d_lam, dgrad);
+    return c->phys == IGAB_PHYS_GETIME ? launch_res_vjp<true>(c, g, dU, dgrad) : launch_res_vjp<false>(c, g, dU, dgrad);
 }
 
 int igab_launch_tangent_transpose(igab_ctx *c, const void *dvals, int prec, const double *dx, double *dy)

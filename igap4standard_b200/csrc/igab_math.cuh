@@ -325,22 +325,123 @@ IGAB_HD igab_tay<N> &operator+=(igab_tay<N> &a, const igab_tay<N> &b)
  * (the expression phys/getime/residual.c:4127-4156 expands).  Its derivative is
  *   d r / d u = 1/2 (H_0/2 + H_1/3 + H_2/4) + diag(rho/dt^2 + c/(2 dt)) on values,
  * H(s) = d2W/du2(m + s h) = sum H_j s^j. */
+/* The derivative components: with E, E_,K, F and G polynomials in s,
+ *   sum_n [S F]_n / (n + 1) = (sum_{n<=3} S_n / (n + 1)) F_0 + (sum_{n<=2} S_n / (n + 2)) F_1
+ * (F = F_0 + s F_1, truncated after the cubic term), and the same for TAU F and TAU G: two static gradients with
+ * averaged stresses.  m, h: the field components of m and h (values unused); r[10 k] is set to 0. */
+template <typename T>
+IGAB_HD void igab_getime_gradient(const T *m, const T *h, const igab_ge_coef &c, T *r)
+{
+    const T is2 = T(IGAB_INV_SQRT2), is3 = T(IGAB_INV_SQRT3), is6 = T(IGAB_INV_SQRT6);
+    igab_ge_point<T> P[2];   /* F, G and averaged stresses of order 0 and 1 */
+    for (int k = 0; k < 3; k++) {
+        for (int J = 0; J < 3; J++) {
+            P[0].F[k][J] = m[10 * k + 1 + J] + (k == J ? T(1) : T(0));
+            P[1].F[k][J] = h[10 * k + 1 + J];
+        }
+        for (int q = 0; q < 6; q++) {
+            P[0].G[k][q] = m[10 * k + 4 + q];
+            P[1].G[k][q] = h[10 * k + 4 + q];
+        }
+    }
+    const T wa[4] = {T(1), T(0.5), T(1.0 / 3.0), T(0.25)}, wb[4] = {T(0.5), T(1.0 / 3.0), T(0.25), T(0)};
+    /* E_0 + s E_1 + s^2 E_2: diagonal entries, and the averaged shear stresses */
+    T e[3][3];
+    for (int I = 0; I < 3; I++)
+        for (int J = I; J < 3; J++) {
+            T x0 = T(0), x1 = T(0), x2 = T(0);
+            for (int k = 0; k < 3; k++) {
+                x0 += P[0].F[k][I] * P[0].F[k][J];
+                x1 += P[0].F[k][I] * P[1].F[k][J] + P[1].F[k][I] * P[0].F[k][J];
+                x2 += P[1].F[k][I] * P[1].F[k][J];
+            }
+            x0 = T(0.5) * (x0 - (I == J ? T(1) : T(0)));
+            x1 = T(0.5) * x1;
+            x2 = T(0.5) * x2;
+            if (I == J) {
+                e[0][I] = x0;
+                e[1][I] = x1;
+                e[2][I] = x2;
+            } else {
+                const int v = 2 + I + J;
+                P[0].d1[v] = T(2) * T(c.p3) * (wa[0] * x0 + wa[1] * x1 + wa[2] * x2);
+                P[1].d1[v] = T(2) * T(c.p3) * (wb[0] * x0 + wb[1] * x1 + wb[2] * x2);
+            }
+        }
+    /* Phi' of (vvol, va, vb), orders 0..3 */
+    T vv[3], va[4], vb[4];
+    for (int j = 0; j < 3; j++) {
+        vv[j] = (e[j][0] + e[j][1] + e[j][2]) * is3;
+        va[j] = (e[j][0] - e[j][1]) * is2;
+        vb[j] = (e[j][0] + e[j][1] - T(2) * e[j][2]) * is6;
+    }
+    va[3] = vb[3] = T(0);
+    T dv[2] = {T(0), T(0)}, da[2] = {T(0), T(0)}, db[2] = {T(0), T(0)};
+    T aa[4], bb[4], ab[4];
+    for (int j = 0; j < 4; j++) {
+        aa[j] = bb[j] = ab[j] = T(0);
+        for (int i = 0; i <= j; i++) {
+            aa[j] += va[i] * va[j - i];
+            bb[j] += vb[i] * vb[j - i];
+            ab[j] += va[i] * vb[j - i];
+        }
+        T s3a = T(0), s3b = T(0);
+        for (int i = 0; i <= j; i++) {
+            s3a += (aa[i] + bb[i]) * va[j - i];
+            s3b += (aa[i] + bb[i]) * vb[j - i];
+        }
+        const T ga = T(-6) * T(c.c36) * ab[j] + T(2) * T(c.c37) * va[j] + T(4) * T(c.c38) * s3a;
+        const T gb = T(3) * T(c.c36) * (bb[j] - aa[j]) + T(2) * T(c.c37) * vb[j] + T(4) * T(c.c38) * s3b;
+        da[0] += wa[j] * ga;
+        db[0] += wa[j] * gb;
+        da[1] += wb[j] * ga;
+        db[1] += wb[j] * gb;
+        if (j < 3) {
+            dv[0] += wa[j] * (T(2) * T(c.p2) * vv[j]);
+            dv[1] += wb[j] * (T(2) * T(c.p2) * vv[j]);
+        }
+    }
+    for (int o = 0; o < 2; o++) {
+        P[o].sig[0] = dv[o] * is3 + da[o] * is2 + db[o] * is6;
+        P[o].sig[1] = dv[o] * is3 - da[o] * is2 + db[o] * is6;
+        P[o].sig[2] = dv[o] * is3 - T(2) * db[o] * is6;
+    }
+    /* TAU: 2 le^2 times the deviator of E_II,K over I */
+    for (int K = 0; K < 3; K++) {
+        T a[3], b[3];
+        for (int I = 0; I < 3; I++) {
+            const int q = igab_idx6(I, K);
+            T x0 = T(0), x1 = T(0), x2 = T(0);
+            for (int k = 0; k < 3; k++) {
+                x0 += P[0].F[k][I] * P[0].G[k][q];
+                x1 += P[0].F[k][I] * P[1].G[k][q] + P[1].F[k][I] * P[0].G[k][q];
+                x2 += P[1].F[k][I] * P[1].G[k][q];
+            }
+            a[I] = wa[0] * x0 + wa[1] * x1 + wa[2] * x2;
+            b[I] = wb[0] * x0 + wb[1] * x1 + wb[2] * x2;
+        }
+        const T ma = (a[0] + a[1] + a[2]) * T(1.0 / 3.0), mb = (b[0] + b[1] + b[2]) * T(1.0 / 3.0);
+        for (int I = 0; I < 3; I++) {
+            P[0].tau[I][K] = T(2) * T(c.p4sq) * (a[I] - ma);
+            P[1].tau[I][K] = T(2) * T(c.p4sq) * (b[I] - mb);
+        }
+    }
+    T r1[30];
+    igab_ge_residual(P[0], r);
+    igab_ge_residual(P[1], r1);
+    for (int i = 0; i < 30; i++) r[i] += r1[i];
+}
+
 template <typename T>
 IGAB_HD void igab_getime_residual(const T *u, const T *u1, const T *u0, const igab_ge_coef &c,
                                   double rho, double cii, double dt, T *r)
 {
-    igab_tay<4> ut[30];
+    T m[30], h[30];
     for (int i = 0; i < 30; i++) {
-        ut[i].c[0] = double((u0[i] + u1[i]) * T(0.5));
-        ut[i].c[1] = double((u[i] - u0[i]) * T(0.5));
-        ut[i].c[2] = 0.0;
-        ut[i].c[3] = 0.0;
+        m[i] = (u0[i] + u1[i]) * T(0.5);
+        h[i] = (u[i] - u0[i]) * T(0.5);
     }
-    igab_ge_point<igab_tay<4>> P;
-    igab_ge_eval(ut, c, P);
-    igab_tay<4> rt[30];
-    igab_ge_residual(P, rt);
-    for (int i = 0; i < 30; i++) r[i] = T(rt[i].c[0] + rt[i].c[1] / 2.0 + rt[i].c[2] / 3.0 + rt[i].c[3] / 4.0);
+    igab_getime_gradient(m, h, c, r);
     for (int k = 0; k < 3; k++)
         r[10 * k] = T(cii) * (u[10 * k] - u0[10 * k]) / T(2.0 * dt) +
                     T(rho) * (u[10 * k] + u0[10 * k] - T(2) * u1[10 * k]) / T(dt * dt);

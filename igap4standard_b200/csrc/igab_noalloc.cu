@@ -69,7 +69,7 @@ extern "C" int igab_residual_noalloc(igab_ctx *ctx, const double *U_host, double
     size_t bytes = (size_t)ctx->ndof * sizeof(double);
     IGAB_CUDA_TRY(cudaMemcpyAsync(dU, U_host, bytes, cudaMemcpyHostToDevice, ctx->stream));
     /* the residual launcher zeroes dR before accumulating, so stale contents never leak */
-    rc = igab_launch_residual(ctx, dU, dR);
+    rc = igab_launch_residual(ctx, dU, dR, false);
     if (rc) return rc;
     IGAB_CUDA_TRY(cudaMemcpyAsync(R_host, dR, bytes, cudaMemcpyDeviceToHost, ctx->stream));
     IGAB_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
