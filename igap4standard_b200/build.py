@@ -28,7 +28,7 @@ CUDA_SOURCES = ["igab_kernels.cu", "igab_tangent_sf.cu", "igab_probes.cu", "igab
                 "igab_batch.cu", "igab_autotune.cu", "igab_noalloc.cu", "igab_density.cu", "igab_krylov.cu",
                 "igab_refine.cu", "igab_newton.cu", "igab_mg.cu", "igab_transient.cu", "igab_periodic.cu"]
 CUDA_HEADERS = ["igab_internal.h", "igab_math.cuh", "igab_device.cuh", "igab_warp_tiles8.inc", "igab_tc.cuh",
-                "igab_reduce.cuh"]
+                "igab_reduce.cuh", "igab_spmv.cuh"]
 
 LIB_CUDA = os.path.join(LIBDIR, "libigap4_b200.so")
 LIB_SUBSET = os.path.join(LIBDIR, "libpetsc_subset.so")

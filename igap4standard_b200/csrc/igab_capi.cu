@@ -384,6 +384,14 @@ int igab_scratch(igab_ctx *c, int kind, size_t bytes, double **out)
     return 0;
 }
 
+void igab_scratch_free(igab_ctx *c)
+{
+    for (double *&p : c->d_scratch) {
+        cudaFree(p);
+        p = nullptr;
+    }
+}
+
 static void free_ctx(igab_ctx *c)
 {
     for (int d = 0; d < 3; d++) {
@@ -395,7 +403,7 @@ static void free_ctx(igab_ctx *c)
     cudaFree(c->d_U); cudaFree(c->d_R); cudaFree(c->d_vals);
     cudaFree(c->d_escale); cudaFree(c->d_lam); cudaFree(c->d_status);
     cudaFree(c->d_dens_part); cudaFree(c->d_HH);
-    cudaFree(c->d_scratch[0]); cudaFree(c->d_scratch[1]);
+    igab_scratch_free(c);
     if (c->scratch_ev) cudaEventDestroy(c->scratch_ev);
     igab_periodic_release(c);
     igab_krylov_release(c);

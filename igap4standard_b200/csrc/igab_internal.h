@@ -256,6 +256,7 @@ enum igab_scratch_kind { IGAB_SCRATCH_TAN = 0, IGAB_SCRATCH_RES = 1 };
 int igab_scratch(igab_ctx *c, int kind, size_t bytes, double **out);
 int igab_scratch_used(igab_ctx *c);
 int igab_scratch_order(igab_ctx *c);
+void igab_scratch_free(igab_ctx *c);
 int igab_launch_exp_scale(igab_ctx *c, const double *dg);
 int igab_launch_adjoint_dRdg(igab_ctx *c, const double *dU, const double *dlam, double *dgrad);
 int igab_launch_tangent_transpose(igab_ctx *c, const void *dvals, int prec, const double *dx, double *dy);

@@ -25,7 +25,7 @@
  */
 #include <cuda_runtime.h>
 #include <vector>
-#include "igab_device.cuh"
+#include "igab_spmv.cuh"
 
 namespace {
 
@@ -42,26 +42,6 @@ struct bcg_state {
 __device__ __forceinline__ bool halted(const bcg_state *S) { return S->stop != 0; }
 __device__ __forceinline__ bool halted_or_half(const bcg_state *S) { return S->stop != 0 || S->half != 0; }
 
-/* the window of control points a row couples to (csr_pos) */
-__device__ __forceinline__ void row_window(const igab_geom &g, long r, int &x0, int &y0, int &z0, int &nxb, int &nyb,
-                                           int &nzb, int &x1, int &y1, int &z1, int &k1)
-{
-    const long cp = r / 3;
-    k1 = (int)(r % 3);
-    z1 = (int)(cp % g.nb[2]);
-    y1 = (int)((cp / g.nb[2]) % g.nb[1]);
-    x1 = (int)(cp / ((long)g.nb[2] * g.nb[1]));
-    x0 = x1 > 2 ? x1 - 2 : 0;
-    y0 = y1 > 2 ? y1 - 2 : 0;
-    z0 = z1 > 2 ? z1 - 2 : 0;
-    const int xe = x1 + 2 < g.nb[0] - 1 ? x1 + 2 : g.nb[0] - 1;
-    const int ye = y1 + 2 < g.nb[1] - 1 ? y1 + 2 : g.nb[1] - 1;
-    const int ze = z1 + 2 < g.nb[2] - 1 ? z1 + 2 : g.nb[2] - 1;
-    nxb = xe - x0 + 1;
-    nyb = ye - y0 + 1;
-    nzb = ze - z0 + 1;
-}
-
 template <typename T>
 __global__ void __launch_bounds__(KV_THREADS) k_spmv(igab_geom g, const T *__restrict__ vals,
                                                      const double *__restrict__ x, double *__restrict__ y,
@@ -71,47 +51,8 @@ __global__ void __launch_bounds__(KV_THREADS) k_spmv(igab_geom g, const T *__res
     const long cp = (long)blockIdx.x * (KV_THREADS / 32) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (3 * cp >= g.ndof) return;   /* warp-uniform */
-    int x0, y0, z0, nxb, nyb, nzb, x1, y1, z1, k1;
-    row_window(g, 3 * cp, x0, y0, z0, nxb, nyb, nzb, x1, y1, z1, k1);
-    const int L = 3 * nzb, total = nxb * nyb * L;   /* L in {9, 12, 15}, total <= 375 */
-    /* lane j < nxb * nyb (<= 25) holds the first column of run j */
-    const long base_own = lane < nxb * nyb ? 3 * cp_index(g, x0 + lane / nyb, y0 + lane % nyb, z0) : 0;
-    /* run = p / L as (p * ceil(2^16 / L)) >> 16, exact for L in {9, 12, 15} and p < 375 */
-    const unsigned invL = (65536u + (unsigned)L - 1u) / (unsigned)L;
-    /* the three rows of the control point share the columns; row k starts k * total later */
-    const T *v0 = vals + g.rowptr[3 * cp], *v1 = v0 + total, *v2 = v1 + total;
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0;
-    /* four 32-entry chunks per pass: every load of the pass is issued before the first
-     * multiply, so a warp keeps 16 loads in flight; the additions keep the chunk order */
-    for (int p0 = 0; p0 < total; p0 += 128) {
-        double xv[4];
-        T w0[4], w1[4], w2[4];
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-            const int p = p0 + 32 * c + lane;
-            const bool in = p < total;
-            const int run = (int)(((unsigned)(in ? p : 0) * invL) >> 16);
-            const long base = __shfl_sync(0xffffffffu, base_own, run);
-            xv[c] = in ? x[base + (p - run * L)] : 0.0;
-            w0[c] = in ? v0[p] : T(0);
-            w1[c] = in ? v1[p] : T(0);
-            w2[c] = in ? v2[p] : T(0);
-        }
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-            if (p0 + 32 * c + lane < total) {
-                a0 += double(w0[c]) * xv[c];
-                a1 += double(w1[c]) * xv[c];
-                a2 += double(w2[c]) * xv[c];
-            }
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        a0 += __shfl_xor_sync(0xffffffffu, a0, o);
-        a1 += __shfl_xor_sync(0xffffffffu, a1, o);
-        a2 += __shfl_xor_sync(0xffffffffu, a2, o);
-    }
+    double a0, a1, a2;
+    spmv_rows<T>(g, vals, x, cp, lane, a0, a1, a2);
     if (lane == 0) {
         y[3 * cp] = a0;
         y[3 * cp + 1] = a1;
