@@ -11,8 +11,8 @@
  *   colour order   natural, mirrored or Gray (igab_colour_at), on the sum of the
  *                  kernels chosen above
  * Batch (igab_batch_autotune):
- *   CTAs per SM of the persistent residual and tangent kernels (1 or as many
- *   as fit), the instance
+ *   CTAs per SM of the persistent residual kernel (1 or as many as fit; the
+ *   tangents run one CTA per work item), the instance
  *   order of the colour-major work list (natural or largest first) and the
  *   colour order.
  * Tile size, CTA count and instance order leave every per-entry summation order
@@ -163,10 +163,8 @@ extern "C" int igab_batch_autotune(igab_batch *b, const double *U_dev, int what,
     }
     IGAB_CUDA_TRY(cudaMalloc(&R.p, (size_t)ndof * sizeof(double)));
     if (what & 14) IGAB_CUDA_TRY(cudaMalloc(&V.p, (size_t)nnz * sizeof(double)));
-    int occ[3] = {0, 0, 0};
-    if ((rc = igab_batch_occupancy_res(&occ[0])) || (rc = igab_batch_occupancy_tan(IGAB_PREC_FP64, &occ[1])) ||
-        (rc = igab_batch_occupancy_tan(IGAB_PREC_FP32, &occ[2])))
-        return rc;
+    int occ[3] = {0, 1, 1};   /* the tangents run one CTA per work item: no CTA count to choose */
+    if ((rc = igab_batch_occupancy_res(&occ[0]))) return rc;
     int cur[4];
     if ((rc = igab_batch_get_schedule(b, &cur[0], &cur[1], &cur[2], &cur[3]))) return rc;
     /* per order: the best CTA count of each timed kernel; the order with the least total wins */

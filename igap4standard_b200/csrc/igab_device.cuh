@@ -118,25 +118,21 @@ __device__ __forceinline__ double elem_scale(const igab_geom &g, int ex, int ey,
 /* ---- persistent batched launches: one work item (a tile of one instance) at a time */
 #define IGAB_BATCH_SPIN (1L << 22)   /* polls (with a 128 ns sleep) before a dependency wait gives up */
 
-/* one thread: wait until every sweep position before `colour` (a position in the
- * batch's colour order) of instance `inst` is complete.  Each wait polls at most B.spin_limit times (128 ns sleep between
- * polls), then sets bit 2 of the status word and moves on; B.hold raises the
- * count that colour 0 of instance 0 must reach, so that the waits on it cannot
- * finish (a host-set test switch that exercises the give-up path). */
-__device__ __forceinline__ void batch_wait_colours(const igab_batch_dev &B, int inst, int colour)
+/* thread c < colour: wait until sweep position c of the batch's colour order is complete for instance `inst` (the
+ * earlier positions are polled side by side).  Each wait polls at most B.spin_limit times (128 ns sleep between
+ * polls), then sets bit 2 of the status word and moves on; B.hold raises the count that colour 0 of instance 0 must
+ * reach, so that the waits on it cannot finish (a host-set test switch that exercises the give-up path). */
+__device__ __forceinline__ void batch_wait_colour(const igab_batch_dev &B, int inst, int c)
 {
-    int *done = B.done + 8 * inst;
-    const int *need = B.need + 8 * inst;
-    for (int c = 0; c < colour; c++) {
-        const int target = need[c] + (inst == 0 && c == 0 ? B.hold : 0);
-        long spins = 0;
-        while (atomicOr(&done[c], 0) < target) {
-            if (++spins > B.spin_limit) {
-                atomicOr(B.status, 2);
-                break;
-            }
-            __nanosleep(128);
+    const volatile int *done = B.done + 8 * inst + c;
+    const int target = B.need[8 * inst + c] + (inst == 0 && c == 0 ? B.hold : 0);
+    long spins = 0;
+    while (*done < target) {
+        if (++spins > B.spin_limit) {
+            atomicOr(B.status, 2);
+            break;
         }
+        __nanosleep(128);
     }
 }
 
@@ -146,39 +142,52 @@ struct batch_slot {
     int pos;          /* position of the colour in the batch's colour order */
 };
 
-/* all threads: fetch the next item, wait until every earlier colour of its
- * instance is complete, stage the instance geometry in shared memory.
- * Returns false when the list is exhausted (block-uniform). */
-__device__ __forceinline__ bool batch_next(const igab_batch_dev &B, batch_slot &sl)
+/* all threads: stage item `it` (its instance's geometry in shared memory), after every earlier colour of its instance */
+__device__ __forceinline__ void batch_stage(const igab_batch_dev &B, batch_slot &sl, bool acquire)
 {
-    if (threadIdx.x == 0) {
-        const int it = atomicAdd(B.counter, 1);
-        sl.item = it;
-        if (it < B.nitems) {
-            const int4 w = B.items[it];
-            sl.inst = w.x;
-            sl.pos = w.y;
-            sl.tile = w.z;
-            sl.colour = w.w;
-            batch_wait_colours(B, w.x, w.y);
-            __threadfence();
-        }
+    if (threadIdx.x < 32) {   /* the barrier below passes the one warp's acquire on to the block */
+        if ((int)threadIdx.x < sl.pos) batch_wait_colour(B, sl.inst, threadIdx.x);
+        __syncwarp();
+        if (acquire && sl.pos > 0) __threadfence();
     }
-    __syncthreads();
-    if (sl.item >= B.nitems) return false;
     const int *src = reinterpret_cast<const int *>(B.geoms + sl.inst);
     int *dst = reinterpret_cast<int *>(&sl.g);
     for (int i = threadIdx.x; i < (int)(sizeof(igab_geom) / sizeof(int)); i += blockDim.x) dst[i] = src[i];
     __syncthreads();
+}
+
+__device__ __forceinline__ void batch_item(const igab_batch_dev &B, batch_slot &sl, int it)
+{
+    const int4 w = B.items[it];
+    sl.inst = w.x;
+    sl.pos = w.y;
+    sl.tile = w.z;
+    sl.colour = w.w;
+}
+
+/* persistent launches: fetch the next item, wait until every earlier colour of its instance is complete, stage the
+ * instance geometry in shared memory.  Returns false when the list is exhausted (block-uniform). */
+__device__ __forceinline__ bool batch_next(const igab_batch_dev &B, batch_slot &sl)
+{
+    if (threadIdx.x == 0) {
+        sl.item = atomicAdd(B.counter, 1);
+        if (sl.item < B.nitems) batch_item(B, sl, sl.item);
+    }
+    __syncthreads();
+    if (sl.item >= B.nitems) return false;
+    batch_stage(B, sl, true);
     return true;
 }
 
-/* all threads, after the item's last global write: publish the finished tile */
-__device__ __forceinline__ void batch_done(const igab_batch_dev &B, const batch_slot &sl)
+/* all threads, after the item's last global write: publish the finished tile (release: the barrier orders the block's
+ * writes before thread 0's fence, which is cumulative) */
+__device__ __forceinline__ void batch_done(const igab_batch_dev &B, const batch_slot &sl, bool release)
 {
-    __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) atomicAdd(&B.done[8 * sl.inst + sl.pos], 1);
+    if (threadIdx.x == 0) {
+        if (release) __threadfence();
+        atomicAdd(&B.done[8 * sl.inst + sl.pos], 1);
+    }
 }
 
 long tiles_of_colour(const igab_geom &g, int TE, int colour)

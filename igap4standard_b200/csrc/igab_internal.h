@@ -234,15 +234,15 @@ int igab_launch_dmma_peak(double *tflops);   /* igab_probes.cu */
 int igab_launch_tan_sf(igab_ctx *c, const double *dU, void *dv, int prec, int tx0, int tx1, bool zero);
 /* persistent batched launches (igab_batch.cu builds the work list) */
 int igab_launch_res_batch(const igab_batch_dev &B, int grid, cudaStream_t s, const double *dU, double *dR);
-int igab_launch_tan_sf_batch(const igab_batch_dev &B, int grid, cudaStream_t s, const double *dU, void *dv, int prec);
+int igab_launch_tan_sf_batch(const igab_batch_dev &B, int item0, int n, cudaStream_t s, const double *dU, void *dv,
+                             int prec);   /* items item0 .. item0 + n - 1, of one colour position */
 int igab_launch_tan_dirichlet_batch(const igab_batch_dev &B, long nd, const int *dinst, const int *drow, void *dv,
                                     int prec, cudaStream_t s);
 /* R = U - g on a list of (global) Dirichlet rows */
 int igab_launch_res_dirichlet_rows(long nd, const int *drow, const double *dg, const double *dU, double *dR,
                                    cudaStream_t s);
-/* CTAs per SM the persistent kernels can hold */
+/* CTAs per SM the persistent residual kernel can hold */
 int igab_batch_occupancy_res(int *per_sm);
-int igab_batch_occupancy_tan(int prec, int *per_sm);
 /* zero the Dirichlet rows of CSR values (rows only) */
 int igab_launch_zero_csr_rows(igab_ctx *c, void *dv, int prec);
 /* the transient tangent (level 0) or history Jacobian (level 1, 2), x tiles [tx0, tx1) */

@@ -856,7 +856,7 @@ __global__ void __launch_bounds__(256, 2) k_res_batch(igab_batch_dev B, const do
         decode_tile(sl.g, 2, sl.colour, sl.tile, T);
         const long off = B.dof_off[sl.inst];
         res_tile<2, false>(sl.g, T, U + off, R + off, S);
-        batch_done(B, sl);
+        batch_done(B, sl, true);
     }
 }
 

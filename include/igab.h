@@ -216,9 +216,9 @@ int igab_autotune(igab_ctx *ctx, const double *U_dev, int what, int reps, igab_t
  * vals[nnz_offsets[i] .. nnz_offsets[i+1]) in its own numbering and AIJ pattern;
  * igab_batch_instance returns its context for pattern queries and parameter
  * changes (then call igab_batch_refresh).  Schedule knobs (the autotuner's search
- * space): CTAs per SM of the residual / FP64 tangent / FP32 tangent persistent
- * kernels (0 = as many as fit) and the instance order of the colour-major work
- * list (0 natural, 1 largest first). */
+ * space): CTAs per SM of the persistent residual (0 = as many as fit; the counts of the FP64
+ * and FP32 tangents are kept and returned, but their kernels run one CTA per tile) and the
+ * instance order of the colour-major work list (0 natural, 1 largest first). */
 typedef struct igab_batch igab_batch;
 int igab_batch_create(const igab_mesh_desc *descs, int n, int device, igab_batch **out);
 int igab_batch_destroy(igab_batch *b);
