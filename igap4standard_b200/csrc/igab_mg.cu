@@ -18,7 +18,7 @@
  * material, boundary tables and (averaged) element scales, whose tangent is assembled
  * at the zero state by the library's own kernels (a preconditioner, so the state it is
  * linearised at only affects the convergence rate).  The coarsest level is solved
- * directly (dense LU with partial pivoting on the host).  Dirichlet rows, identity rows
+ * directly (its inverse, below).  Dirichlet rows, identity rows
  * of every level's tangent, are masked out of the restricted residuals and of the
  * prolonged corrections, which keeps the V-cycle symmetric.
  *
@@ -42,7 +42,12 @@
  * On meshes of some ten thousand dofs a solve is bound by the number of its short kernels, not by their bytes: the
  * smoother's vector updates ride on its products (9 kernels per level and V-cycle instead of 30, 6 products instead of
  * 7), the V-cycle is one graph launch, and a Gram-Schmidt step keeps its coefficients on the device and is read once.
- * 16^3, 108 GMRES iterations of three Newton steps: 50.4 -> 18.9 ms (465 -> 175 us per iteration).
+ * 16^3, 108 GMRES iterations of three Newton steps: 50.4 -> 18.9 ms (465 -> 175 us per iteration), and 18.9 -> 13.7 ms
+ * (127 us) with the next kernel launched and its matrix rows and tables loaded under the one before (mg_launch), the
+ * Gram-Schmidt products of all vectors side by side, and blocks for the dofs there are (8^3: 6.5 -> 4.6 ms, 32^3, 185
+ * iterations: 110.5 -> 95.2 ms).  What is left at 16^3 is 7 fine products of 9 us (6 us of them latency: three passes
+ * of loads on 1.2 waves of blocks) and some 25 other kernels of 3-5 us.  Left out: more blocks per SM by fewer
+ * registers (spills, 14.0-19.6 ms), rows cut at whole runs of columns (half the instructions, no faster, 32^3 101.6).
  * Measured and rejected: the smoothing operators stored in half precision (64^3: 4.58 ->
  * 4.36 ms per GMRES iteration, but one more iteration per solve; no gain per Newton step).
  */
@@ -51,6 +56,7 @@
 #include <cstring>
 #include <vector>
 #include <cuda_runtime.h>
+#include <type_traits>
 #include "igab_internal.h"
 #include "igab_reduce.cuh"
 #include "igab_spmv.cuh"
@@ -59,6 +65,8 @@ namespace {
 
 #define MG_THREADS 256
 #define MG_BLOCKS 296
+#define MG_ALL 4096            /* control points up to which a product loads its rows whole, before the wait (mg_spmv) */
+#define MG_SPMV 128            /* block of the smoother's products: small, so that a coarse level spreads over the SMs */
 #define MG_MAX_LEVELS 8
 #define MG_DEGREE 3            /* Chebyshev degree per smoothing */
 #define MG_POWER_ITERS 12      /* power iterations for lmax of D^-1 K */
@@ -106,6 +114,32 @@ __global__ void k_mg_diag_inv(igab_geom g, const void *__restrict__ vals, int pr
 
 #define MG_LOOP(i, n) for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < (n); i += (long)gridDim.x * blockDim.x)
 
+/* Programmatic dependent launch.  The kernels of a V-cycle and of a Gram-Schmidt step follow one another in a stream
+ * and take 2-7 us each, so a kernel is launched (mg_launch) while the one before it still runs: it loads what no kernel
+ * of the solve writes (the matrix, the tables), then mg_wait() returns when the kernel before has completed and its
+ * writes are visible, and lets the next one be launched.  A kernel of the chain therefore starts only after the one
+ * two before it has completed.  Vectors are read after mg_wait() and through pointers without __restrict__, which
+ * keeps them off the read-only path. */
+__device__ __forceinline__ void mg_wait()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <class... K, class... A>
+void mg_launch(void (*k)(K...), dim3 grid, int block, cudaStream_t st, A... a)
+{
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&cfg, k, K(a)...);   /* an error stays for the callers' cudaGetLastError() */
+}
+
 /* d = s * dinv * r */
 __global__ void k_mg_jac(long n, const double *__restrict__ dinv, const double *__restrict__ r, double s,
                          double *__restrict__ d)
@@ -134,37 +168,47 @@ __global__ void k_mg_start(long n, const double *__restrict__ in, const double *
  *   MG_LAST_POST   t = K d: x += d + d', the residual after the last step is not needed
  * d' goes to another vector than d, whose neighbours the other rows still read. */
 enum { MG_STEP = 0, MG_LAST_PRE = 1, MG_RESID = 2, MG_LAST_POST = 3 };
-template <typename T, int OP>
-__global__ void __launch_bounds__(MG_THREADS) k_mg_spmv(igab_geom g, const T *__restrict__ vals,
-                                                        const double *__restrict__ in, const double *__restrict__ b,
-                                                        const double *__restrict__ dinv,
-                                                        const unsigned char *__restrict__ mask, double a, double c,
-                                                        int first, double *__restrict__ x, double *__restrict__ r,
-                                                        double *__restrict__ dn)
+template <typename T, int OP, bool ALL>
+__global__ void __launch_bounds__(MG_SPMV, ALL ? 4 : 8) k_mg_spmv(igab_geom g, const T *__restrict__ vals, const double *in,
+                                                     const double *b, const double *__restrict__ dinv,
+                                                     const unsigned char *__restrict__ mask, double a, double c,
+                                                     int first, double *x, double *r, double *dn)
 {
-    const long cp = (long)blockIdx.x * (MG_THREADS / 32) + (threadIdx.x >> 5);
+    const long cp = (long)blockIdx.x * (MG_SPMV / 32) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (3 * cp >= g.ndof) return;   /* warp-uniform */
-    double a0, a1, a2;
-    spmv_rows<T>(g, vals, in, cp, lane, a0, a1, a2);
-    if (lane >= 3) return;
     const long i = 3 * cp + lane;
-    const double t = lane == 0 ? a0 : (lane == 1 ? a1 : a2);
+    spmv_part<T> P;
+    if (ALL) spmv_load<T>(g, vals, cp, lane, P);
+    double di = 0.0, u = 0.0, ro = 0.0, xo = 0.0, s[3];
+    int dirichlet = 0;
+    if (lane < 3) {
+        di = dinv[i];
+        if (OP == MG_LAST_PRE) dirichlet = mask[i];
+    }
+    mg_wait();
+    if (lane < 3) {
+        ro = OP == MG_RESID ? b[i] : r[i];
+        if (OP != MG_RESID) u = in[i];
+        if (OP != MG_RESID && !first) xo = x[i];
+    }
+    if (ALL) spmv_mult<T>(P, in, lane, s);
+    else spmv_rows<T>(g, vals, in, cp, lane, s[0], s[1], s[2]);
+    if (lane >= 3) return;
+    const double ri = ro - (lane == 0 ? s[0] : (lane == 1 ? s[1] : s[2]));
     if (OP == MG_RESID) {
-        const double ri = b[i] - t;
         r[i] = ri;
-        dn[i] = a * dinv[i] * ri;
+        dn[i] = a * di * ri;
         return;
     }
-    const double d = in[i], ri = r[i] - t;
-    const double xn = first ? d : x[i] + d;
+    const double xn = first ? u : xo + u;
     if (OP == MG_LAST_POST) {
-        x[i] = xn + (a * d + c * dinv[i] * ri);
+        x[i] = xn + (a * u + c * di * ri);
         return;
     }
     x[i] = xn;
-    r[i] = OP == MG_LAST_PRE && mask[i] ? 0.0 : ri;
-    if (OP == MG_STEP) dn[i] = a * d + c * dinv[i] * ri;
+    r[i] = OP == MG_LAST_PRE && dirichlet ? 0.0 : ri;
+    if (OP == MG_STEP) dn[i] = a * u + c * di * ri;
 }
 
 /* r = b - t */
@@ -200,17 +244,41 @@ struct mg_dirs_dev {
 };
 
 /* xf += P xc off the Dirichlet rows (tensor product of the three 1-D prolongations, per displacement component) */
-__global__ void k_mg_prolong(mg_dirs_dev D, const double *__restrict__ xc, const unsigned char *__restrict__ mask,
-                             double *__restrict__ xf)
+__global__ void __launch_bounds__(MG_THREADS) k_mg_prolong(mg_dirs_dev D, const double *xc,
+                                                           const unsigned char *__restrict__ mask, double *xf)
 {
-    const long n = 3L * D.nbf[0] * D.nbf[1] * D.nbf[2];
-    MG_LOOP(i, n)
-    {
-        if (mask[i]) continue;
-        const long f = i / 3;
-        const int k = (int)(i - 3 * f);
-        const int iz = (int)(f % D.nbf[2]), iy = (int)((f / D.nbf[2]) % D.nbf[1]), ix = (int)(f / ((long)D.nbf[2] * D.nbf[1]));
-        double s = 0.0;
+    const long n = 3L * D.nbf[0] * D.nbf[1] * D.nbf[2], i = blockIdx.x * (long)MG_THREADS + threadIdx.x;
+    if (i >= n) return;
+    const int dirichlet = mask[i];
+    const long f = i / 3;
+    const int k = (int)(i - 3 * f);
+    const int iz = (int)(f % D.nbf[2]), iy = (int)((f / D.nbf[2]) % D.nbf[1]), ix = (int)(f / ((long)D.nbf[2] * D.nbf[1]));
+    /* the first two of each direction's points (there are no more with every other knot removed) before the wait */
+    int j[3][2];
+    double w[3][2];
+#pragma unroll
+    for (int d = 0; d < 3; d++)
+#pragma unroll
+        for (int a = 0; a < 2; a++) {
+            const int o = (d == 0 ? ix : (d == 1 ? iy : iz)) * D.kp[d] + a;
+            const bool in = a < D.kp[d];
+            j[d][a] = in ? D.p_idx[d][o] : 0;
+            w[d][a] = in ? D.p_w[d][o] : 0.0;
+        }
+    mg_wait();   /* also where nothing is added: each grid of the chain has to wait somewhere */
+    if (dirichlet) return;
+    const double old = xf[i];
+    double s = 0.0;
+    if (D.kp[0] <= 2 && D.kp[1] <= 2 && D.kp[2] <= 2) {
+#pragma unroll
+        for (int a = 0; a < 2; a++)
+#pragma unroll
+            for (int b = 0; b < 2; b++)
+#pragma unroll
+                for (int c = 0; c < 2; c++)
+                    s += w[0][a] * w[1][b] * w[2][c] *
+                         xc[3 * (((long)j[0][a] * D.nbc[1] + j[1][b]) * D.nbc[2] + j[2][c]) + k];
+    } else {
         for (int a = 0; a < D.kp[0]; a++) {
             const double wa = D.p_w[0][ix * D.kp[0] + a];
             const int ja = D.p_idx[0][ix * D.kp[0] + a];
@@ -221,34 +289,51 @@ __global__ void k_mg_prolong(mg_dirs_dev D, const double *__restrict__ xc, const
                     s += wab * D.p_w[2][iz * D.kp[2] + c] * xc[3 * (jab + D.p_idx[2][iz * D.kp[2] + c]) + k];
             }
         }
-        xf[i] += s;
     }
+    xf[i] = old + s;
 }
 
 /* b = r = P^T rf, zero on the Dirichlet rows, d = s dinv b (the coarse level's right-hand side and first direction) */
-__global__ void __launch_bounds__(MG_THREADS) k_mg_restrict(mg_dirs_dev D, const double *__restrict__ rf,
+__global__ void __launch_bounds__(MG_THREADS) k_mg_restrict(mg_dirs_dev D, const double *rf,
                                                             const unsigned char *__restrict__ mask,
-                                                            const double *__restrict__ dinv, double s,
-                                                            double *__restrict__ b, double *__restrict__ r,
-                                                            double *__restrict__ d)
+                                                            const double *__restrict__ dinv, double s, double *b,
+                                                            double *r, double *d)
 {
     const long nc = (long)D.nbc[0] * D.nbc[1] * D.nbc[2];
     const long j = (long)blockIdx.x * (MG_THREADS / 32) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (j >= nc) return;   /* warp-uniform */
     const int jz = (int)(j % D.nbc[2]), jy = (int)((j / D.nbc[2]) % D.nbc[1]), jx = (int)(j / ((long)D.nbc[2] * D.nbc[1]));
+    const long i = 3 * j + lane;
+    const double di = lane < 3 ? dinv[i] : 0.0;
+    const int dirichlet = lane < 3 ? mask[i] : 0;
     double v[3] = {0.0, 0.0, 0.0};
+    bool waited = false;
     /* a lane takes every 32nd of the (a, e) pairs of fine lines, then a fixed shuffle tree */
-    for (int p = lane; p < D.kr[0] * D.kr[1]; p += 32) {
-        const int a = p / D.kr[1], e = p - a * D.kr[1];
-        const double wab = D.r_w[0][jx * D.kr[0] + a] * D.r_w[1][jy * D.kr[1] + e];
-        const long iab = ((long)D.r_idx[0][jx * D.kr[0] + a] * D.nbf[1] + D.r_idx[1][jy * D.kr[1] + e]) * D.nbf[2];
-        for (int c = 0; c < D.kr[2]; c++) {
-            const double w = wab * D.r_w[2][jz * D.kr[2] + c];
-            const double *u = rf + 3 * (iab + D.r_idx[2][jz * D.kr[2] + c]);
-            v[0] += w * u[0];
-            v[1] += w * u[1];
-            v[2] += w * u[2];
+    for (int p0 = 0; p0 < D.kr[0] * D.kr[1]; p0 += 32) {
+        const int p = p0 + lane, a = p / D.kr[1], e = p - a * D.kr[1];
+        const bool in = p < D.kr[0] * D.kr[1];
+        const double wab = in ? D.r_w[0][jx * D.kr[0] + a] * D.r_w[1][jy * D.kr[1] + e] : 0.0;
+        const long iab = in ? ((long)D.r_idx[0][jx * D.kr[0] + a] * D.nbf[1] + D.r_idx[1][jy * D.kr[1] + e]) * D.nbf[2] : 0;
+        for (int c0 = 0; c0 < D.kr[2]; c0 += 4) {
+            double w[4];
+            int o[4];
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                const bool inc = c0 + c < D.kr[2];
+                w[c] = inc ? wab * D.r_w[2][jz * D.kr[2] + c0 + c] : 0.0;
+                o[c] = inc ? D.r_idx[2][jz * D.kr[2] + c0 + c] : -1;
+            }
+            if (!waited) mg_wait();   /* warp-uniform */
+            waited = true;
+#pragma unroll
+            for (int c = 0; c < 4; c++)
+                if (in && o[c] >= 0) {
+                    const double *u = rf + 3 * (iab + o[c]);
+                    v[0] += w[c] * u[0];
+                    v[1] += w[c] * u[1];
+                    v[2] += w[c] * u[2];
+                }
         }
     }
 #pragma unroll
@@ -256,11 +341,10 @@ __global__ void __launch_bounds__(MG_THREADS) k_mg_restrict(mg_dirs_dev D, const
 #pragma unroll
         for (int k = 0; k < 3; k++) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
     if (lane >= 3) return;
-    const long i = 3 * j + lane;
-    const double u = mask[i] ? 0.0 : (lane == 0 ? v[0] : (lane == 1 ? v[1] : v[2]));
+    const double u = dirichlet ? 0.0 : (lane == 0 ? v[0] : (lane == 1 ? v[1] : v[2]));
     b[i] = u;
     r[i] = u;
-    d[i] = s * dinv[i] * u;
+    d[i] = s * di * u;
 }
 
 } /* namespace */
@@ -533,14 +617,24 @@ struct mg_cheb {
 template <int OP>
 void mg_spmv(igab_mg *m, mg_level &L, cudaStream_t st, const double *in, double a, double c, int first, double *dn)
 {
-    const unsigned nblk = (unsigned)((L.n / 3 + MG_THREADS / 32 - 1) / (MG_THREADS / 32));
+    const unsigned nblk = (unsigned)((L.n / 3 + MG_SPMV / 32 - 1) / (MG_SPMV / 32));
     const igab_geom g = L.ctx->geom();
-    if (L.prec == IGAB_PREC_FP64)
-        k_mg_spmv<double, OP><<<nblk, MG_THREADS, 0, st>>>(g, (const double *)L.vals, in, L.b, L.dinv, L.mask, a, c, first,
-                                                          L.x, L.r, dn);
-    else
-        k_mg_spmv<float, OP><<<nblk, MG_THREADS, 0, st>>>(g, (const float *)L.vals, in, L.b, L.dinv, L.mask, a, c, first,
-                                                         L.x, L.r, dn);
+    const auto go = [&](auto *vals, auto all) {
+        using T = std::remove_const_t<std::remove_pointer_t<decltype(vals)>>;
+        mg_launch(k_mg_spmv<T, OP, decltype(all)::value>, nblk, MG_SPMV, st, g, vals, in, L.b, L.dinv, L.mask, a, c, first,
+                  L.x, L.r, dn);
+    };
+    /* up to about two waves of blocks (148 SMs x 16 warps) the rows are loaded whole under the kernel before; beyond,
+     * the registers that takes cost more than the wait: 1,000 points (8^3) 4.7 against 5.2 us, the 2,744 of 12^3 within
+     * a 24^3 solve 39.3 against 40.8 ms, but 5,832 (16^3) 15.5 against 13.7 ms and 32^3 120 against 95 ms a solve */
+    const bool all = L.n / 3 <= MG_ALL;
+    if (L.prec == IGAB_PREC_FP64) {
+        if (all) go((const double *)L.vals, std::true_type());
+        else go((const double *)L.vals, std::false_type());
+    } else {
+        if (all) go((const float *)L.vals, std::true_type());
+        else go((const float *)L.vals, std::false_type());
+    }
     m->launches++;
 }
 
@@ -565,12 +659,12 @@ __global__ void k_mg_gj_init(int n, const double *__restrict__ A, double *__rest
 /* Gauss-Jordan step k in place (row-major A), from the old pivot row / column (row, col);
  * writes row / column k + 1 of the result into (nrow, ncol) for the next step.  Each
  * entry is computed by one thread from the old values only. */
-__global__ void k_mg_gj_step(int n, int k, double *__restrict__ A, const double *__restrict__ row,
-                             const double *__restrict__ col, double *__restrict__ nrow, double *__restrict__ ncol,
-                             int *__restrict__ flag)
+__global__ void k_mg_gj_step(int n, int k, double *A, const double *row,
+                             const double *col, double *nrow, double *ncol, int *flag)
 {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= n || j >= n) return;
+    mg_wait();
+    const int t = blockIdx.x * MG_THREADS + threadIdx.x, i = t / n, j = t - i * n;   /* n <= MG_COARSE_DOF */
+    if (i >= n) return;
     const double p = col[k];
     if (i == k && j == k && !(p > 0.0 && isfinite(p))) *flag = 1;
     const double ip = 1.0 / p;
@@ -583,14 +677,24 @@ __global__ void k_mg_gj_step(int n, int k, double *__restrict__ A, const double 
     if (j == k + 1) ncol[i] = v;
 }
 
-/* x = Ainv b: one warp per row, lane-strided partial sums then a fixed shuffle tree */
-__global__ void k_mg_gemv(long n, const double *__restrict__ Ai, const double *__restrict__ b, double *__restrict__ x)
+/* x = Ainv b: one warp per row (the first 24 x 32 of its entries before the wait), lane-strided partial sums then a
+ * fixed shuffle tree */
+__global__ void __launch_bounds__(128) k_mg_gemv(long n, const double *__restrict__ Ai, const double *b, double *x)
 {
     const long r = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (r >= n) return;
-    double s = 0.0;
-    for (long j = lane; j < n; j += 32) s += Ai[r * n + j] * b[j];
+    const double *row = Ai + r * n;
+    double w[24], s = 0.0;
+#pragma unroll
+    for (int c = 0; c < 24; c++) w[c] = 32 * c + lane < n ? row[32 * c + lane] : 0.0;
+    mg_wait();
+    double v[24];
+#pragma unroll
+    for (int c = 0; c < 24; c++) v[c] = 32 * c + lane < n ? b[32 * c + lane] : 0.0;
+#pragma unroll
+    for (int c = 0; c < 24; c++) s += w[c] * v[c];
+    for (long j = 768 + lane; j < n; j += 32) s += row[j] * b[j];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane == 0) x[r] = s;
@@ -603,7 +707,7 @@ int vcycle(igab_mg *m, int l, cudaStream_t st)
     mg_level &L = m->L[l];
     if (l == m->nlev - 1) {
         if (m->direct && m->dev_inv) {
-            k_mg_gemv<<<(unsigned)((L.n + 7) / 8), 256, 0, st>>>(L.n, m->inv, L.b, L.x);
+            mg_launch(k_mg_gemv, (unsigned)((L.n + 3) / 4), 128, st, L.n, m->inv, L.b, L.x);
             m->launches++;
         } else if (m->direct) {
             IGAB_CUDA_TRY(cudaMemcpyAsync(m->h_vec, L.b, (size_t)L.n * sizeof(double), cudaMemcpyDeviceToHost, st));
@@ -628,11 +732,12 @@ int vcycle(igab_mg *m, int l, cudaStream_t st)
     /* coarse correction with the Dirichlet rows of both levels masked (symmetric; a coarse x is zero on them, as its
      * right-hand side is and the operators have unit rows and columns there) */
     const mg_dirs_dev D = dirs_view(C);
-    k_mg_restrict<<<(unsigned)((C.n / 3 + MG_THREADS / 32 - 1) / (MG_THREADS / 32)), MG_THREADS, 0, st>>>(D, L.r, C.mask, C.dinv, 1.0 / mg_cheb(C.lmax).theta, C.b, C.r, C.d);
+    mg_launch(k_mg_restrict, (unsigned)((C.n / 3 + MG_THREADS / 32 - 1) / (MG_THREADS / 32)), MG_THREADS, st, D, L.r, C.mask,
+              C.dinv, 1.0 / mg_cheb(C.lmax).theta, C.b, C.r, C.d);
     m->launches++;
     int rc = vcycle(m, l + 1, st);
     if (rc) return rc;
-    k_mg_prolong<<<MG_BLOCKS, MG_THREADS, 0, st>>>(D, C.x, L.mask, L.x);
+    mg_launch(k_mg_prolong, (unsigned)((L.n + MG_THREADS - 1) / MG_THREADS), MG_THREADS, st, D, C.x, L.mask, L.x);
     m->launches++;
     /* r = b - K x, then the same smoother again */
     d = L.d;
@@ -797,10 +902,10 @@ int mg_build(igab_ctx *c, igab_mg *m)
             if (e == cudaSuccess) {
                 k_mg_dense<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, cc->d_rowptr, dcols, B.own_vals, m->inv);
                 k_mg_gj_init<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, m->inv, m->gj, m->gj + n);
-                const dim3 grid((unsigned)((n + 15) / 16), (unsigned)((n + 15) / 16)), blk(16, 16);
+                const unsigned blocks = (unsigned)(((long)n * n + MG_THREADS - 1) / MG_THREADS);
                 for (int k = 0; k < n; k++) {
                     double *rk = m->gj + (size_t)(k & 1) * 2 * n, *nx = m->gj + (size_t)((k + 1) & 1) * 2 * n;
-                    k_mg_gj_step<<<grid, blk, 0, st>>>(n, k, m->inv, rk, rk + n, nx, nx + n, m->gj_flag);
+                    mg_launch(k_mg_gj_step, blocks, MG_THREADS, st, n, k, m->inv, rk, rk + n, nx, nx + n, m->gj_flag);
                 }
                 e = cudaGetLastError();
             }
@@ -863,63 +968,67 @@ int igab_mg_levels(igab_ctx *c, int *levels)
 
 namespace {
 
-/* partial sums of V_i . w, i < k (V_i = V + i n), per block into part[i][RD_BLOCKS]; the warps' sums meet once, after
- * all vectors (one barrier, not two per vector) */
-__global__ void __launch_bounds__(RD_THREADS) k_md_partial(long n, const double *__restrict__ V, int k,
-                                                           const double *__restrict__ w, double *part)
+/* partial sums of V_i . w for the four i from 4 blockIdx.y (V_i = V + i n, i < k), per block into part[i][RD_BLOCKS] */
+__global__ void __launch_bounds__(RD_THREADS) k_md_partial(long n, const double *V, int k, const double *w, double *part)
 {
-    __shared__ double red[GM_RESTART + 1][RD_THREADS / 32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const long t0 = blockIdx.x * (long)RD_THREADS + threadIdx.x, step = (long)RD_BLOCKS * RD_THREADS;
-    for (int i0 = 0; i0 < k; i0 += 4) {
-        double s[4] = {0.0, 0.0, 0.0, 0.0};
-        for (long t = t0; t < n; t += step) {
-            const double x = w[t];
+    __shared__ double red[4][RD_THREADS / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, i0 = 4 * blockIdx.y;
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    mg_wait();
+    MG_LOOP(t, n)
+    {
+        const double x = w[t];
 #pragma unroll
-            for (int i = 0; i < 4; i++)
-                if (i0 + i < k) s[i] += V[(size_t)(i0 + i) * n + t] * x;
-        }
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            if (i0 + i >= k) break;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) s[i] += __shfl_xor_sync(0xffffffffu, s[i], o);
-            if (lane == 0) red[i0 + i][warp] = s[i];
-        }
+        for (int i = 0; i < 4; i++)
+            if (i0 + i < k) s[i] += V[(size_t)(i0 + i) * n + t] * x;
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int i = 0; i < 4; i++) s[i] += __shfl_xor_sync(0xffffffffu, s[i], o);
+    if (lane < 4) red[lane][warp] = lane == 0 ? s[0] : (lane == 1 ? s[1] : (lane == 2 ? s[2] : s[3]));
     __syncthreads();
-    if (threadIdx.x < k) {
-        double s = 0.0;
-        for (int q = 0; q < RD_THREADS / 32; q++) s += red[threadIdx.x][q];
-        part[(size_t)threadIdx.x * RD_BLOCKS + blockIdx.x] = s;
+    if (threadIdx.x < 4 && i0 + threadIdx.x < k) {
+        double q = 0.0;
+#pragma unroll
+        for (int e = 0; e < RD_THREADS / 32; e++) q += red[threadIdx.x][e];
+        part[(size_t)(i0 + threadIdx.x) * RD_BLOCKS + blockIdx.x] = q;
     }
 }
 
-/* out[i] = sum of part[i][0..RD_BLOCKS) in a fixed order, one block per i */
-__global__ void __launch_bounds__(RD_THREADS) k_md_finish(const double *part, double *out)
+/* the sum of part[0..nb) in a fixed order, in every thread of the block (nb <= RD_BLOCKS <= 2 RD_THREADS) */
+__device__ __forceinline__ double md_sum(const double *part, int nb)
 {
     __shared__ double red[RD_THREADS / 32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    double s = 0.0;
-    for (int b = threadIdx.x; b < RD_BLOCKS; b += RD_THREADS) s += part[(size_t)blockIdx.x * RD_BLOCKS + b];
+    const int t = threadIdx.x;
+    double s = t < nb ? part[t] : 0.0;
+    if (t + RD_THREADS < nb) s += part[t + RD_THREADS];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) red[warp] = s;
+    if ((t & 31) == 0) red[t >> 5] = s;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int q = 0; q < RD_THREADS / 32; q++) t += red[q];
-        out[blockIdx.x] = t;
-    }
+    double q = 0.0;
+#pragma unroll
+    for (int e = 0; e < RD_THREADS / 32; e++) q += red[e];
+    return q;
+}
+static_assert(RD_BLOCKS <= 2 * RD_THREADS, "two partial sums per thread");
+
+/* out[i] = sum of part[i][0..nb), one block per i */
+__global__ void __launch_bounds__(RD_THREADS) k_md_finish(const double *part, int nb, double *out)
+{
+    mg_wait();
+    const double q = md_sum(part + (size_t)blockIdx.x * RD_BLOCKS, nb);
+    if (threadIdx.x == 0) out[blockIdx.x] = q;
 }
 
 /* w -= sum_{i<k} h_i V_i (h on the device); with part: the blocks' partial sums of w . w */
-__global__ void __launch_bounds__(RD_THREADS) k_md_update(long n, const double *__restrict__ V, int k,
-                                                          const double *__restrict__ h, double *__restrict__ w,
+__global__ void __launch_bounds__(RD_THREADS) k_md_update(long n, const double *V, int k, const double *h, double *w,
                                                           double *part)
 {
     __shared__ double red[RD_THREADS / 32];
     double q = 0.0;
+    mg_wait();
     MG_LOOP(t, n)
     {
         double s = w[t];
@@ -940,19 +1049,12 @@ __global__ void __launch_bounds__(RD_THREADS) k_md_update(long n, const double *
     }
 }
 
-/* *nn = w . w from the partial sums (every block adds them up in the same order), v = w / ||w|| */
-__global__ void __launch_bounds__(RD_THREADS) k_md_scale(long n, const double *__restrict__ w, const double *part,
-                                                         double *__restrict__ nn, double *__restrict__ v)
+/* *nn = w . w from the nb partial sums (every block adds them up in the same order), v = w / ||w|| */
+__global__ void __launch_bounds__(RD_THREADS) k_md_scale(long n, const double *w, const double *part, int nb, double *nn,
+                                                         double *v)
 {
-    __shared__ double red[RD_THREADS / 32];
-    double s = 0.0;
-    for (int b = threadIdx.x; b < RD_BLOCKS; b += RD_THREADS) s += part[b];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-    __syncthreads();
-    double q = 0.0;
-    for (int i = 0; i < RD_THREADS / 32; i++) q += red[i];
+    mg_wait();
+    const double q = md_sum(part, nb);
     if (blockIdx.x == 0 && threadIdx.x == 0) *nn = q;
     const double inv = q > 0.0 ? 1.0 / sqrt(q) : 0.0;
     MG_LOOP(t, n) v[t] = inv * w[t];
@@ -969,23 +1071,28 @@ __global__ void k_md_combine(long n, const double *__restrict__ V, int k, const 
     }
 }
 
+/* the blocks of a vector kernel: no more than the vector fills */
+int md_blocks(long n) { return (int)std::min<long>(RD_BLOCKS, (n + RD_THREADS - 1) / RD_THREADS); }
+
 /* out = V[0..k)^T w, on the device */
 void mdot(igab_mg *m, cudaStream_t st, long n, const double *V, int k, const double *w, double *out)
 {
-    k_md_partial<<<RD_BLOCKS, RD_THREADS, 0, st>>>(n, V, k, w, m->mpart);
-    k_md_finish<<<k, RD_THREADS, 0, st>>>(m->mpart, out);
+    const int nb = md_blocks(n);
+    mg_launch(k_md_partial, dim3((unsigned)nb, (unsigned)((k + 3) / 4)), RD_THREADS, st, n, V, k, w, m->mpart);
+    mg_launch(k_md_finish, (unsigned)k, RD_THREADS, st, m->mpart, nb, out);
     m->launches += 2;
 }
 
 /* the V-cycle as the preconditioner: L[0].x = M r.  Its kernels are replayed from a graph, captured after each build of
- * the hierarchy (not with the host LU, which reads and writes in between). */
+ * the hierarchy (not with the host LU, which reads and writes in between, nor on the legacy stream, which cannot be
+ * captured). */
 int precond(igab_mg *m, const double *r)
 {
     mg_level &F = m->L[0];
     cudaStream_t st = F.ctx->stream;
     k_mg_start<<<MG_BLOCKS, MG_THREADS, 0, st>>>(F.n, r, F.dinv, 1.0 / mg_cheb(F.lmax).theta, F.b, F.r, F.d);
     m->launches++;
-    if (m->direct && !m->dev_inv) return vcycle(m, 0, st);
+    if ((m->direct && !m->dev_inv) || st == cudaStreamLegacy) return vcycle(m, 0, st);
     if (!m->vexec) {
         const int l0 = m->launches;
         cudaGraph_t gr = nullptr;
@@ -1061,7 +1168,7 @@ int solve_gmres(igab_mg *m, igab_ctx *c, const void *vals, int prec, const doubl
 {
     cudaStream_t st = c->stream;
     const long n = c->ndof;
-    const int mr = GM_RESTART;
+    const int mr = GM_RESTART, nb = md_blocks(n);
     double *V = m->kv, *w = V + (size_t)(mr + 1) * n, *r = w + n;
     const double *t = m->L[0].x;   /* the preconditioner's result */
     /* device: h of the first and of the second projection, ||w||^2; h_md receives the three */
@@ -1089,10 +1196,10 @@ int solve_gmres(igab_mg *m, igab_ctx *c, const void *vals, int prec, const doubl
             /* CGS2: h = V^T w, w -= V h, twice; the next basis vector w / ||w||; one read of the coefficients */
             double *part = m->mpart;
             mdot(m, st, n, V, j + 1, w, dev_h);
-            k_md_update<<<RD_BLOCKS, RD_THREADS, 0, st>>>(n, V, j + 1, dev_h, w, nullptr);
+            mg_launch(k_md_update, nb, RD_THREADS, st, n, V, j + 1, dev_h, w, nullptr);
             mdot(m, st, n, V, j + 1, w, dev_h2);
-            k_md_update<<<RD_BLOCKS, RD_THREADS, 0, st>>>(n, V, j + 1, dev_h2, w, part);
-            k_md_scale<<<RD_BLOCKS, RD_THREADS, 0, st>>>(n, w, part, dev_nn, V + (size_t)(j + 1) * n);
+            mg_launch(k_md_update, nb, RD_THREADS, st, n, V, j + 1, dev_h2, w, part);
+            mg_launch(k_md_scale, nb, RD_THREADS, st, n, w, part, nb, dev_nn, V + (size_t)(j + 1) * n);
             IGAB_CUDA_TRY(cudaGetLastError());
             IGAB_CUDA_TRY(cudaMemcpyAsync(m->h_md, dev_h, (size_t)(2 * mr + 3) * sizeof(double), cudaMemcpyDeviceToHost, st));
             IGAB_CUDA_TRY(cudaStreamSynchronize(st));
