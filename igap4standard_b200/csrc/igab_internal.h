@@ -234,6 +234,10 @@ int igab_launch_dmma_peak(double *tflops);   /* igab_probes.cu */
 int igab_launch_tan_sf(igab_ctx *c, const double *dU, void *dv, int prec, int tx0, int tx1, bool zero);
 /* persistent batched launches (igab_batch.cu builds the work list) */
 int igab_launch_res_batch(const igab_batch_dev &B, int grid, cudaStream_t s, const double *dU, double *dR);
+/* element layers ex0 .. ex1 - 1 through the scratch ke of `ring` layers, and the rows they complete; igab_tan_sf_steps
+ * gives the scratch (null: not this way) and the layers per call, and igab_scratch_used follows the last call */
+int igab_tan_sf_steps(igab_ctx *c, int prec, int *step, int *ring, double **ke);
+int igab_launch_tan_sf_layers(igab_ctx *c, const double *dU, void *dv, int prec, double *ke, int ex0, int ex1, int ring);
 int igab_launch_tan_sf_batch(const igab_batch_dev &B, int item0, int n, cudaStream_t s, const double *dU, void *dv,
                              int prec);   /* items item0 .. item0 + n - 1, of one colour position */
 int igab_launch_tan_dirichlet_batch(const igab_batch_dev &B, long nd, const int *dinst, const int *drow, void *dv,

@@ -22,6 +22,7 @@
  * X_q[v][(a,k)] = sum_m dv/du_{k,m} N_a^{m}(q), a rank-12 update per point
  * plus a geometric block shared by the three displacement components.
  */
+#include <algorithm>
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include "igab_internal.h"
@@ -1032,11 +1033,33 @@ int launch_tangent_t(igab_ctx *c, const double *dU, T *dv)
     return 0;
 }
 
-/* x-slab boundaries (odd tile coordinates, increasing) of the host-pointer tangent:
- * slabs of 8 tiles, then 4, 2, 2 and 1 (or 2) tiles at the end, so that the rows
- * finished last, whose download cannot overlap any compute, are few.  None below
- * 12 tiles. */
-int slab_bounds(int ntx, int *b)
+/* x-slab boundaries (odd tile coordinates, increasing) of the host-pointer tangent's tiles.  The bus takes 174 ns (FP64)
+ * or 87 ns (FP32) for an element's values and the static assembly 78 ns, so the first slab is small, for the download
+ * to start early, the next ones double up to 8 tiles, and the last ones halve again, as the rows finished last overlap
+ * no compute.  A slab is at least q tiles long, so that each of its eight launches has about a block per SM.  None below
+ * 3 q tiles.  48 x 40 x 40 FP64 18.4 -> 16.7 ms, 16 x 48 x 48 9.9 -> 8.7 (FP32 11.4 -> 11.4, 6.5 -> 6.1); with twice the
+ * q 21.5 and 9.9. */
+#define SLAB_TILES 1184
+int slab_bounds(const int ne[3], int *b)
+{
+    const int ntx = (ne[0] + 1) / 2;
+    const long plane = (long)((ne[1] + 1) / 2) * ((ne[2] + 1) / 2);
+    const int q = (int)std::max(2L, (SLAB_TILES + plane - 1) / plane / 2 * 2), cap = std::max({8, q, ntx / 24 * 2});
+    int n = 0, x = q - 1, step = q;
+    if (ntx < 3 * q) return 0;
+    b[n++] = x;
+    while (ntx - x >= 2 * q && n < IGAB_MAX_SLABS - 1) {
+        x += std::max(q, std::min(step, (ntx - x) / 4 * 2));
+        b[n++] = x;
+        step = std::min(2 * step, cap);
+    }
+    return n;
+}
+
+/* the same where the assembly is the slower part (transient: 145 ns an element, one block per SM): slabs of 8 tiles,
+ * then 4, 2, 2 and 1 (or 2) tiles at the end.  None below 12 tiles.  With the bounds above instead, 32 x 32 x 40 FP32
+ * took 10.6 ms against 8.1. */
+int slab_bounds_late(int ntx, int *b)
 {
     if (ntx < 12) return 0;
     int tmp[IGAB_MAX_SLABS], n = 0;
@@ -1063,7 +1086,37 @@ int launch_tangent_slabs_t(igab_ctx *c, const double *dU, T *dv, long *row_end, 
     const int ntx = (c->ne[0] + 1) / 2;
     int b[IGAB_MAX_SLABS];
     const bool ranged = c->phys == IGAB_PHYS_GETIME || (sizeof(T) == 8 ? c->tan_kernel == 1 : c->tan32_kernel == 1);
-    const int nb = ranged ? slab_bounds(ntx, b) : 0;
+    const int prec = sizeof(T) == 8 ? IGAB_PREC_FP64 : IGAB_PREC_FP32;
+    int step = 0, ring = 0, rc = 0;
+    double *ke = nullptr;
+    if (ranged && (rc = igab_tan_sf_steps(c, prec, &step, &ring, &ke))) return rc;
+    if (ke) {   /* layers of elements through the scratch, an event after every m-th step */
+        igab_mark(c, 3);
+        const long plane = 3L * c->nb[1] * c->nb[2];
+        const int steps = (c->ne[0] + step - 1) / step, m = (steps + IGAB_MAX_SLABS - 1) / IGAB_MAX_SLABS;
+        const int l0 = c->last_launches;
+        int n = 0, nd = 0;
+        long r0 = 0;
+        for (int i = 0; i < steps; i++) {
+            const int ex0 = i * step, ex1 = std::min(c->ne[0], ex0 + step);
+            if ((rc = igab_launch_tan_sf_layers(c, dU, dv, prec, ke, ex0, ex1, ring))) return rc;
+            if (i < steps - 1 && (i + 1) % m) continue;
+            if (i == steps - 1) igab_mark(c, 4);
+            const long r1 = i < steps - 1 ? ex1 * plane : c->ndof;
+            const int ld = c->last_launches;
+            if ((rc = launch_tan_dirichlet<T>(c, g, dv, r0, r1))) return rc;
+            nd += c->last_launches - ld;
+            if (!c->slab_ev[n]) IGAB_CUDA_TRY(cudaEventCreateWithFlags(&c->slab_ev[n], cudaEventDisableTiming));
+            IGAB_CUDA_TRY(cudaEventRecord(c->slab_ev[n], c->stream));
+            row_end[n++] = r0 = r1;
+        }
+        c->nvol_tan = c->last_launches - l0 - nd;
+        igab_mark(c, 5);
+        c->ev_tan = c->profiling;
+        *nslab = n;
+        return igab_scratch_used(c);
+    }
+    const int nb = !ranged ? 0 : (c->phys == IGAB_PHYS_GETIME ? slab_bounds_late(ntx, b) : slab_bounds(c->ne, b));
     for (int i = 0; i <= nb; i++)
         if (!c->slab_ev[i]) IGAB_CUDA_TRY(cudaEventCreateWithFlags(&c->slab_ev[i], cudaEventDisableTiming));
     IGAB_CUDA_TRY(cudaMemsetAsync(dv, 0, (size_t)c->nnz * sizeof(T), c->stream));

@@ -42,6 +42,7 @@
  * of the code under run-time slots and phases (54 instead of 85 KB of code, +2.5 ms); padding of the element
  * matrices against bank conflicts (no change).
  */
+#include <algorithm>
 #include <cuda_runtime.h>
 #include <type_traits>
 #include "igab_device.cuh"
@@ -56,6 +57,8 @@ namespace {
  * (transient 8^3 1,207 -> 109, 16^3 1,216 -> 695); three meshes on three streams, which fill one another's gaps:
  * 12^3 369 -> 215 us each, 16^3 476 -> 503, 20^3 648 -> 972. */
 #define SF_ELEM_MAX 4096
+#define SF_STEP 1184                     /* elements of a step of the host entry point: four of two blocks per SM */
+#define SF_LAYER_MAX (SF_ELEM_MAX / 3)   /* its largest layer: a step and the two layers before it fit */
 
 /* ---- derivative components m = 0..8: x y z xx xy xz yy yz zz; class = (kx, ky) in the order
  * 0:(0,0) 1:(0,1) 2:(0,2) 3:(1,0) 4:(1,1) 5:(2,0) */
@@ -793,9 +796,18 @@ struct sf_tile_io {
     }
 };
 /* ... or every gridDim-th element of the mesh into a scratch array [element][6 pairs][729] */
+/* Where the scratch holds a layer of elements: layer ex at ex % ring, for the layers of one launch, from `first` on,
+ * which wrap once at most (a division per element cost 3% at 8^3) */
+struct sf_ring {
+    int wrap, below, above;
+    sf_ring(int first, int ring) : wrap(first / ring * ring + ring), below(ring - wrap), above(-wrap) {}
+    __device__ __forceinline__ int slot(int ex) const { return ex + (ex < wrap ? below : above); }
+};
+
 struct sf_elem_io {
     double *ke;
     long e, ne;
+    const sf_ring &ring;
     __device__ __forceinline__ bool next(const igab_geom &g, sf_elem &E)
     {
         e += gridDim.x;
@@ -808,7 +820,7 @@ struct sf_elem_io {
                                         int s2, int tid)
     {
         /* rows 0 bring the pairs (0,0) (0,1) (0,2), rows 1 (1,1) (1,2), rows 2 (2,2): slot s_l, l >= k */
-        double *o = ke + (((long)E.ex * g.ne[1] + E.ey) * g.ne[2] + E.ez) * 4374 + (k == 0 ? 0 : (k == 1 ? 3 : 5)) * 729;
+        double *o = ke + (((long)ring.slot(E.ex) * g.ne[1] + E.ey) * g.ne[2] + E.ez) * 4374 + (k == 0 ? 0 : (k == 1 ? 3 : 5)) * 729;
         for (int l = k; l < 3; l++, o += 729) {
             const double *K = SF_KSLOT(S, l == 0 ? s0 : (l == 1 ? s1 : s2));
             for (int i = tid; i < 729; i += SF_THR) o[i] = K[i];
@@ -910,15 +922,16 @@ __global__ void __launch_bounds__(SF_THR, NR == 1 ? 2 : 1) k_tan_sf(igab_geom g,
     sf_run<NR>(g, C, io, U, S);
 }
 
-/* every element matrix of a mesh into a scratch array */
+/* the matrices of elements e0 .. ne - 1 into a scratch array */
 template <int NR>
 __global__ void __launch_bounds__(SF_THR, NR == 1 ? 2 : 1) k_tan_sf_elem(igab_geom g, sf_coef C,
                                                                          const double *__restrict__ U,
-                                                                         double *__restrict__ ke, long ne)
+                                                                         double *__restrict__ ke, long e0, long ne,
+                                                                         sf_ring ring)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     sf_smem<NR> &S = *reinterpret_cast<sf_smem<NR> *>(smem_raw);
-    sf_elem_io io = {ke, (long)blockIdx.x - (long)gridDim.x, ne};
+    sf_elem_io io = {ke, e0 + (long)blockIdx.x - (long)gridDim.x, ne, ring};
     sf_run<NR>(g, C, io, U, S);
 }
 
@@ -928,9 +941,9 @@ __global__ void __launch_bounds__(SF_THR, NR == 1 ? 2 : 1) k_tan_sf_elem(igab_ge
  * tile) and in the same precision, so the values equal theirs bit for bit. */
 template <typename T>
 __global__ void __launch_bounds__(384) k_tan_gather(igab_geom g, const double *__restrict__ ke, T *__restrict__ vals,
-                                                    int order)
+                                                    int order, int cp0, sf_ring ring)
 {
-    const int cp = blockIdx.x, s = threadIdx.x;
+    const int cp = cp0 + blockIdx.x, s = threadIdx.x;
     const int z = cp % g.nb[2], y = (cp / g.nb[2]) % g.nb[1], x = cp / (g.nb[2] * g.nb[1]);
     const int x0 = max(x - 2, 0), y0 = max(y - 2, 0), y1 = min(y + 2, g.nb[1] - 1);
     const int z0 = max(z - 2, 0), z1 = min(z + 2, g.nb[2] - 1);
@@ -954,10 +967,11 @@ __global__ void __launch_bounds__(384) k_tan_gather(igab_geom g, const double *_
 #pragma unroll 1
     for (int kp = 0; kp < 8; kp++) {
         const int col = igab_colour_at(order, kp), px = col >> 2, py = (col >> 1) & 1, pz = col & 1;
-        for (int ex = px ? lo[0][1] : lo[0][0]; ex < (px ? hi[0][1] : hi[0][0]); ex++)
+        for (int ex = px ? lo[0][1] : lo[0][0]; ex < (px ? hi[0][1] : hi[0][0]); ex++) {
+            const int slot = ring.slot(ex);
             for (int ey = py ? lo[1][1] : lo[1][0]; ey < (py ? hi[1][1] : hi[1][0]); ey++)
                 for (int ez = pz ? lo[2][1] : lo[2][0]; ez < (pz ? hi[2][1] : hi[2][0]); ez++) {
-                    const double *K = ke + (((long)ex * g.ne[1] + ey) * g.ne[2] + ez) * 4374;
+                    const double *K = ke + (((long)slot * g.ne[1] + ey) * g.ne[2] + ez) * 4374;
                     const int ax = x - ex, ay = y - ey, az = z - ez, bx = cx - ex, by = cy - ey, bz = cz - ez;
                     const int i = (3 * ax + bx) * 81 + (3 * ay + by) * 9 + 3 * az + bz;
                     const int it = (3 * bx + ax) * 81 + (3 * by + ay) * 9 + 3 * bz + az;
@@ -968,6 +982,7 @@ __global__ void __launch_bounds__(384) k_tan_gather(igab_geom g, const double *_
 #pragma unroll
                     for (int k = 0; k < 3; k++) acc[k] += T(k == l ? v[k] + w : v[k]);
                 }
+        }
     }
     T *o = vals + r0 + s;
 #pragma unroll
@@ -1003,23 +1018,39 @@ int sm_count(int device)
     return cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && n > 0 ? n : 148;
 }
 
+/* element layers ex0 .. ex1 - 1 into the scratch (of `ring` layers), then the rows they complete: those of the control
+ * points x = ex0 .. ex1 - 1, of all the rest with the last layer */
 template <typename T, int NR>
-int launch_sf(igab_ctx *c, const igab_geom &g, const sf_coef &C, const double *dU, T *dv, int tx0, int tx1, bool zero)
+int launch_sf_layers(igab_ctx *c, const igab_geom &g, const sf_coef &C, const double *dU, T *dv, double *ke, int ex0,
+                     int ex1, int ring)
 {
     const size_t sm = sizeof(sf_smem<NR>);
-    double *ke = nullptr;
+    const long layer = (long)g.ne[1] * g.ne[2], ne = (ex1 - ex0) * layer, cap = (NR == 1 ? 2L : 1L) * sm_count(c->device);
+    const int plane = g.nb[1] * g.nb[2], x1 = ex1 == g.ne[0] ? g.nb[0] : ex1;
+    IGAB_CUDA_TRY(cudaFuncSetAttribute(k_tan_sf_elem<NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    k_tan_sf_elem<NR><<<(unsigned)(ne < cap ? ne : cap), SF_THR, sm, c->stream>>>(g, C, dU, ke, ex0 * layer, ex1 * layer,
+                                                                                  sf_ring(ex0, ring));
+    k_tan_gather<T><<<(unsigned)((x1 - ex0) * plane), 384, 0, c->stream>>>(g, ke, dv, c->colour_order, ex0 * plane,
+                                                                         sf_ring(std::max(ex0 - 2, 0), ring));
+    c->last_launches += 2;
+    IGAB_CUDA_TRY(cudaGetLastError());
+    return 0;
+}
+
+/* tx0 .. tx1: tiles along x; with ke: element layers tx0 .. tx1 through that scratch (igab_launch_tan_sf_layers) */
+template <typename T, int NR>
+int launch_sf(igab_ctx *c, const igab_geom &g, const sf_coef &C, const double *dU, T *dv, int tx0, int tx1, bool zero,
+              double *ke = nullptr, int ring = 0)
+{
+    if (ke) return launch_sf_layers<T, NR>(c, g, C, dU, dv, ke, tx0, tx1, ring);
+    const size_t sm = sizeof(sf_smem<NR>);
     if (tx0 == 0 && tx1 == (g.ne[0] + 1) / 2 && c->nel <= SF_ELEM_MAX) {
         int rc = igab_scratch(c, IGAB_SCRATCH_TAN, (size_t)c->nel * 4374 * sizeof(double), &ke);
         if (rc) return rc;
     }
     if (ke) {
-        IGAB_CUDA_TRY(cudaFuncSetAttribute(k_tan_sf_elem<NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        const long cap = (NR == 1 ? 2L : 1L) * sm_count(c->device);
-        k_tan_sf_elem<NR><<<(unsigned)(c->nel < cap ? c->nel : cap), SF_THR, sm, c->stream>>>(g, C, dU, ke, c->nel);
-        k_tan_gather<T><<<(unsigned)c->ncp, 384, 0, c->stream>>>(g, ke, dv, c->colour_order);
-        c->last_launches += 2;
-        IGAB_CUDA_TRY(cudaGetLastError());
-        return igab_scratch_used(c);
+        const int rc = launch_sf_layers<T, NR>(c, g, C, dU, dv, ke, 0, g.ne[0], g.ne[0]);
+        return rc ? rc : igab_scratch_used(c);
     }
     if (zero) {
         IGAB_CUDA_TRY(cudaMemsetAsync(dv, 0, (size_t)c->nnz * sizeof(T), c->stream));
@@ -1040,19 +1071,9 @@ int launch_sf(igab_ctx *c, const igab_geom &g, const sf_coef &C, const double *d
 
 } /* namespace */
 
-int igab_launch_tan_sf(igab_ctx *c, const double *dU, void *dv, int prec, int tx0, int tx1, bool zero)
+/* the coefficients of the transient integrand's derivative by the newest (0) or an older level; g gets its weights */
+static sf_coef sf_coef_getime(igab_geom &g, int level)
 {
-    const igab_geom g = c->geom();
-    if (c->phys == IGAB_PHYS_GETIME) return igab_launch_tan_getime_level(c, dU, dv, prec, 0, tx0, tx1, zero);
-    const sf_coef C = sf_coef_ge(g);
-    return prec == IGAB_PREC_FP64 ? launch_sf<double, 1>(c, g, C, dU, (double *)dv, tx0, tx1, zero)
-                                  : launch_sf<float, 1>(c, g, C, dU, (float *)dv, tx0, tx1, zero);
-}
-
-int igab_launch_tan_getime_level(igab_ctx *c, const double *dU, void *dv, int prec, int level, int tx0, int tx1,
-                                 bool zero)
-{
-    igab_geom g = c->geom();
     if (level == 1) {          /* d r / d u1 */
         const double w[4] = {0.5, 0.25, 1.0 / 6.0, 0.125};
         for (int j = 0; j < 4; j++) g.tw[j] = w[j];
@@ -1070,8 +1091,54 @@ int igab_launch_tan_getime_level(igab_ctx *c, const double *dU, void *dv, int pr
     C.al = 1.0 / C.r00;
     C.ga = 1.0 / C.r11;
     C.be = -C.r01 * C.al * C.ga;
-    return prec == IGAB_PREC_FP64 ? launch_sf<double, 2>(c, g, C, dU, (double *)dv, tx0, tx1, zero)
-                                  : launch_sf<float, 2>(c, g, C, dU, (float *)dv, tx0, tx1, zero);
+    return C;
+}
+
+static int launch_sf_any(igab_ctx *c, const double *dU, void *dv, int prec, int level, int tx0, int tx1, bool zero,
+                         double *ke = nullptr, int ring = 0)
+{
+    igab_geom g = c->geom();
+    if (c->phys == IGAB_PHYS_GETIME) {
+        const sf_coef C = sf_coef_getime(g, level);
+        return prec == IGAB_PREC_FP64 ? launch_sf<double, 2>(c, g, C, dU, (double *)dv, tx0, tx1, zero, ke, ring)
+                                      : launch_sf<float, 2>(c, g, C, dU, (float *)dv, tx0, tx1, zero, ke, ring);
+    }
+    const sf_coef C = sf_coef_ge(g);
+    return prec == IGAB_PREC_FP64 ? launch_sf<double, 1>(c, g, C, dU, (double *)dv, tx0, tx1, zero, ke, ring)
+                                  : launch_sf<float, 1>(c, g, C, dU, (float *)dv, tx0, tx1, zero, ke, ring);
+}
+
+int igab_launch_tan_sf(igab_ctx *c, const double *dU, void *dv, int prec, int tx0, int tx1, bool zero)
+{
+    return launch_sf_any(c, dU, dv, prec, 0, tx0, tx1, zero);
+}
+
+int igab_launch_tan_getime_level(igab_ctx *c, const double *dU, void *dv, int prec, int level, int tx0, int tx1,
+                                 bool zero)
+{
+    return launch_sf_any(c, dU, dv, prec, level, tx0, tx1, zero);
+}
+
+/* The host entry point's tangent goes through the scratch in steps of some layers of elements along x, so that the
+ * download starts after the first: a step has some four waves of elements, and the scratch holds a step and the two
+ * layers before it, which its first rows need too.  An element costs 119 ns this way and 78 in large slabs of tiles, but
+ * a launch of few tiles takes 133 us however few they are, and the bus 174 ns (FP64) or 87 (FP32) per element: layers
+ * too large for the scratch, or half that for FP32, go by tiles.  Whole call: 24 x 21 x 26 FP64 4.0 -> 2.8 ms, FP32 3.5
+ * -> 2.3, transient 4.5 -> 3.3; 16^3 1.54 -> 1.21; 40 x 36 x 36 FP64 12.1 -> 9.6, but FP32 7.9 by tiles, 8.7 this way. */
+int igab_tan_sf_steps(igab_ctx *c, int prec, int *step, int *ring, double **ke)
+{
+    *ke = nullptr;
+    const long layer = (long)c->ne[1] * c->ne[2];
+    if (layer > (prec == IGAB_PREC_FP64 ? SF_LAYER_MAX : SF_LAYER_MAX / 2)) return 0;
+    const long s = std::max(1L, SF_STEP / layer), r = c->nel <= SF_ELEM_MAX ? c->ne[0] : SF_ELEM_MAX / layer;
+    *ring = (int)r;
+    *step = (int)(r < c->ne[0] ? std::min(s, r - 2) : s);
+    return igab_scratch(c, IGAB_SCRATCH_TAN, (size_t)(r * layer) * 4374 * sizeof(double), ke);
+}
+
+int igab_launch_tan_sf_layers(igab_ctx *c, const double *dU, void *dv, int prec, double *ke, int ex0, int ex1, int ring)
+{
+    return launch_sf_any(c, dU, dv, prec, 0, ex0, ex1, false, ke, ring);
 }
 
 template <typename T>

@@ -95,3 +95,14 @@ def test_streams_and_captures(built, make):
     g.replay()
     torch.cuda.synchronize()
     assert torch.equal(R, R0) and torch.equal(V, V0)
+
+
+@pytest.mark.parametrize("ne,prec", [((9, 12, 13), "fp64"), ((9, 36, 37), "fp64"), ((11, 26, 26), "fp32"),
+                                     ((13, 37, 37), "fp64"), ((14, 26, 27), "fp32")])
+def test_host_steps_and_slabs(built, ne, prec):
+    """The host tangent by steps of layers through a ring of layers (all of a small mesh, many, three of 1,332 elements,
+    six of 676) and, with larger layers, by slabs of tiles: the values of the one-pass tangent."""
+    A, U = _static(ne)
+    _, _, V = _device(A, U, prec)
+    for _ in range(2):
+        assert np.array_equal(V.cpu().numpy(), A.tangent(U, prec))
