@@ -16,7 +16,8 @@
  * shuffles (reduce-scatter across the 4 lanes of a direction) and one
  * shared-memory step across the two warps.
  *
- * Tangent (src/snesiga_Tangent.c:99-190): per element, 256 threads.  With
+ * Tangent on the FMA pipe (src/snesiga_Tangent.c:99-190; a kernel option, the default is
+ * igab_tangent_sf.cu): per element, 256 threads.  With
  * the energy written as W = Phi(v(u)) over 12 variables (igab_math.cuh),
  *   K_e = sum_q w_q [ X_q^T Phi''_q X_q + blockdiag(Gamma_q) ],
  * X_q[v][(a,k)] = sum_m dv/du_{k,m} N_a^{m}(q), a rank-12 update per point
@@ -344,8 +345,11 @@ __device__ __forceinline__ void res_tile(const igab_geom &g, const tile_t &T, co
     }
 }
 
+/* Three blocks per SM at 80 registers (some 200 B of spills) against two at 128: 48^3 on three streams 829 -> 812 us,
+ * 64^3 1958 -> 1922, and 30^3 through the scratch 216 -> 203; four (64 registers) 1001, 2435 and 310.  The components
+ * one after the other, to need fewer registers, gained nothing. */
 template <int TE, bool GT>
-__global__ void __launch_bounds__(256, GT ? 1 : 2) k_res_volume(igab_geom g, const double *__restrict__ U,
+__global__ void __launch_bounds__(256, GT ? 1 : (TE == 2 ? 3 : 2)) k_res_volume(igab_geom g, const double *__restrict__ U,
                                                     double *__restrict__ R, int colour)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -370,7 +374,7 @@ struct res_elem_smem {
     double Re[4][81];
 };
 template <bool GT, bool VJP>
-__global__ void __launch_bounds__(256, GT ? 1 : 2) k_res_elem(igab_geom g, const double *__restrict__ U, double *__restrict__ out,
+__global__ void __launch_bounds__(256, GT ? 1 : 3) k_res_elem(igab_geom g, const double *__restrict__ U, double *__restrict__ out,
                                                   const double *__restrict__ lam, long ne)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
