@@ -22,7 +22,7 @@
  * of every level's tangent, are masked out of the restricted residuals and of the
  * prolonged corrections, which keeps the V-cycle symmetric.
  *
- * Smoother: Chebyshev polynomial of degree 3 in D^-1 K on [lmax / 10, 1.1 lmax], lmax
+ * Smoother: Chebyshev polynomial of degree 6 in D^-1 K on [1.1 lmax / 100, 1.1 lmax], lmax
  * estimated by power iteration; the same polynomial before and after the coarse
  * correction, so the V-cycle is a symmetric preconditioner and CG applies.
  *
@@ -46,7 +46,8 @@
  * (127 us) with the next kernel launched and its matrix rows and tables loaded under the one before (mg_launch), the
  * Gram-Schmidt products of all vectors side by side, and blocks for the dofs there are (8^3: 6.5 -> 4.6 ms, 32^3, 185
  * iterations: 110.5 -> 95.2 ms).  What is left at 16^3 is 7 fine products of 9 us (6 us of them latency: three passes
- * of loads on 1.2 waves of blocks) and some 25 other kernels of 3-5 us.  Left out: more blocks per SM by fewer
+ * of loads on 1.2 waves of blocks) and some 25 other kernels of 3-5 us (with the smoother's degree 3 of that time; now
+ * 6, and 45 iterations of 200 us).  Left out: more blocks per SM by fewer
  * registers (spills, 14.0-19.6 ms), rows cut at whole runs of columns (half the instructions, no faster, 32^3 101.6).
  * Measured and rejected: the smoothing operators stored in half precision (64^3: 4.58 ->
  * 4.36 ms per GMRES iteration, but one more iteration per solve; no gain per Newton step).
@@ -68,7 +69,8 @@ namespace {
 #define MG_ALL 4096            /* control points up to which a product loads its rows whole, before the wait (mg_spmv) */
 #define MG_SPMV 128            /* block of the smoother's products: small, so that a coarse level spreads over the SMs */
 #define MG_MAX_LEVELS 8
-#define MG_DEGREE 3            /* Chebyshev degree per smoothing */
+#define MG_DEGREE 6            /* Chebyshev degree per smoothing */
+#define MG_RATIO 100.0         /* largest to smallest eigenvalue of its interval (mg_cheb) */
 #define MG_POWER_ITERS 12      /* power iterations for lmax of D^-1 K */
 #define GM_RESTART 50          /* GMRES restart length */
 #define MG_COARSE_DOF 1200     /* the coarsest level is solved directly below this size */
@@ -595,13 +597,19 @@ int estimate_lmax(igab_mg *m, mg_level &L)
     return 0;
 }
 
-/* the Chebyshev recurrence on [lmax / 10, 1.1 lmax]: the first direction is dinv r / theta, step i makes the next one
+/* The interval is wide and the degree high, as the operator is of fourth order: an error of half the coarse mesh's
+ * resolution has 2^-4 or less of lmax, and the rediscretised coarse operator corrects the modes near that poorly.
+ * GMRES of three Newton steps at 8^3 / 16^3 / 32^3 (ms; iterations at 16^3): degree 3, ratio 10: 4.6 / 13.8 / 95.2
+ * (108); degree 3, ratio 30: 16^3 11.7, 32^3 79.7 (91); degree 4, 30: 11.0, 78.6 (73); degree 6: ratio 40 10.4, 80.2,
+ * 80 2.8 / 9.3 / 70.7 (47), 120 3.3 / 8.7 / 68.2 (44), 200 4.1 / 8.9 / 64.6; degree 8: ratio 100 2.8 / 8.7 / 71.7 (35),
+ * 200 3.7 / 8.6 / 65.1; degree 10, 200: 3.5 / 8.8 / 67.4; degree 2, 10: 15.0, 92.2 (140).
+ * The Chebyshev recurrence on [1.1 lmax / ratio, 1.1 lmax]: the first direction is dinv r / theta, step i makes the next one
  * a d + c dinv r */
 struct mg_cheb {
     double theta, a[MG_DEGREE], c[MG_DEGREE];
     explicit mg_cheb(double lmax)
     {
-        const double hi = 1.1 * lmax, lo = hi / 10.0, delta = 0.5 * (hi - lo);
+        const double hi = 1.1 * lmax, lo = hi / MG_RATIO, delta = 0.5 * (hi - lo);
         theta = 0.5 * (hi + lo);
         const double sigma = theta / delta;
         double rho = 1.0 / sigma;
