@@ -11,9 +11,9 @@ cube with interior knots perturbed by +-0.1h (seed 1), (lambda, mu, l) =
 uniform in +-1e-3 (seed 0).
 
   value     FP64 path, inputs resident in HBM, ms per assembly (device events)
-  mixed     FP32-built tangent + FP64 residual, same timing
+  mixed     FP32 tangent values + FP64 residual, same timing
   e2e       FP64 path through the host-pointer C ABI (U in, R and CSR values out)
-  roofline  tangent volume kernel against the measured FP64 FMA peak
+  roofline  tangent volume kernel against the measured FP64 tensor-pipe peak
   cpu_baseline  the reference's own assembly (oracle/_ref) on the host cores
 
 Usage: python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
@@ -41,11 +41,11 @@ METRIC = "Newton-step assembly ms & adjoint grads/s at 64^3, mixed vs FP64, 1xB2
 GE_RESIDUAL_INTEGRAND_FLOPS = 758
 TAN_ALG_FLOPS = 64 * 2 * (30 * 81 * 10 + 81 * 81 * 10)
 RES_ALG_FLOPS = 64 * (2 * (27 * 30 + 27 * 30) + 270 + GE_RESIDUAL_INTEGRAND_FLOPS)
-# flops the tangent kernel executes per element on the tensor path: 66 upper 8x8 tiles
-# x 12 variables per point, plus 10 upper 8x8 tiles of the geometric block x 6 U / V rows per point
-TAN_EXEC_FLOPS = 64 * 2 * (66 * 64 * 12 + 10 * 64 * 6)
-# DRAM bytes per element of the FP64 tangent kernel (ncu, 32^3 colour launch: 243.12 MB / 4,096)
-TAN64_DRAM_BYTES_PER_ELEMENT = 243.12e6 / 4096
+# flops the tangent kernel executes per element on the tensor path: about 1,900 m8n8k4 products of the
+# sum-factorised contraction (the point matrices run on the FP64 FMA pipe beside them)
+TAN_EXEC_FLOPS = 1900 * 2 * 8 * 8 * 4
+# DRAM bytes per element of the FP64 tangent kernel (ncu, 40^3 colour launch: 295.39 + 260.75 MB / 8,000)
+TAN64_DRAM_BYTES_PER_ELEMENT = 556.14e6 / 8000
 
 
 def parse():
@@ -773,44 +773,37 @@ def run_ours(args):
     # ---- roofline of the dominant kernel (tangent volume, 8 colour launches per step)
     tan_ms = k64[2]
     nlaunch = max(k64[5], 1)
-    achieved = nel * TAN_ALG_FLOPS / (tan_ms * 1e-3) / 1e12
-    executed = nel * TAN_EXEC_FLOPS / (tan_ms * 1e-3) / 1e12
-    # DRAM traffic of the FP64 tangent kernel from one ncu capture of a 32^3 colour launch
-    # (dram__bytes_read.sum + dram__bytes_write.sum = 151.08 MB + 92.04 MB for 4,096
+    achieved = nel * TAN_EXEC_FLOPS / (tan_ms * 1e-3) / 1e12
+    dense = nel * TAN_ALG_FLOPS / (tan_ms * 1e-3) / 1e12
+    # DRAM traffic of the FP64 tangent kernel from one ncu capture of a 40^3 colour launch
+    # (dram__bytes_read.sum + dram__bytes_write.sum = 295.39 MB + 260.75 MB for 8,000
     # elements), scaled to a launch of this mesh by its elements (the traffic is the CSR
     # read-modify-write of each element matrix, so it grows with the element count)
     traffic = round(TAN64_DRAM_BYTES_PER_ELEMENT * nel / nlaunch)
     roofline = {"bound": "tensor", "pipe": "FP64 tensor (mma.sync m8n8k4 f64) + FP64 FMA", "achieved": round(achieved, 3),
                 "peak": round(peak64, 3),
                 "unit": "TFLOP/s", "frac": round(achieved / peak64, 4), "traffic": traffic,
-                "traffic_source": "ncu dram bytes of one 32^3 colour launch (4,096 elements), scaled per element",
-                "kernel": "k_tan_dmma", "avg_launch_ms": round(tan_ms / nlaunch, 3),
-                "flops_per_launch": nel * TAN_ALG_FLOPS / nlaunch,
-                "flops_definition": "algorithmic B^T D B per element = 64*2*(30*81*10+81*81*10) (effective: the "
-                                    "kernel executes %d flops per element)" % TAN_EXEC_FLOPS,
-                "executed_tflops": round(executed, 3),
+                "traffic_source": "ncu dram bytes of one 40^3 colour launch (8,000 elements), scaled per element",
+                "kernel": "k_tan_sf<double, 1>", "avg_launch_ms": round(tan_ms / nlaunch, 3),
+                "flops_per_launch": nel * TAN_EXEC_FLOPS / nlaunch,
+                "flops_definition": "executed on the tensor path per element (%d: sum-factorised contraction; a dense "
+                                    "B^T D B, 64*2*(30*81*10+81*81*10) = %d, is not formed)" % (TAN_EXEC_FLOPS,
+                                                                                               TAN_ALG_FLOPS),
+                "dense_equivalent_tflops": round(dense, 3),
                 "peak_fp64_fma": round(peak64_fma, 3), "peak_fp64_dmma": round(peak64_dmma, 3),
-                "executed_frac_of_dmma_peak": round(executed / peak64_dmma, 4),
+                "executed_frac_of_dmma_peak": round(achieved / peak64_dmma, 4),
                 "peak_source": "measured, burst: the larger of the FP64 FMA probe (igab_fma_peak) and the FP64 "
                                "tensor-pipe probe (igab_dmma_peak, back-to-back mma.sync m8n8k4 f64); "
                                "MEASURED_PEAKS.json has no FP64 figure"}
     res_tf = nel * RES_ALG_FLOPS / (k64[0] * 1e-3) / 1e12 if k64[0] > 0 else None
-    # FP32 (mixed) tangent on tcgen05: per element 768 curvature rows in chunks of 32 (about 25 chunks,
-    # 8 MMAs M128 x N96 x K8 each); the geometric block runs on the FP32 FMA pipe
-    tc_exec_per_el = 25 * 8 * 2 * 128 * 96 * 8
+    # the mixed path's tangent: the same FP64 kernel, values rounded to FP32 at the store
     tan32_ms = k32[2]
     nl32 = max(k32[5], 1)
-    roofline_mixed = {"bound": "tensor", "pipe": "TF32 tcgen05 (hi/lo split, FP32 accumulation)",
-                      "kernel": "k_tan_tc32<2>", "avg_launch_ms": round(tan32_ms / nl32, 3),
-                      "achieved": round(nel * TAN_ALG_FLOPS / (tan32_ms * 1e-3) / 1e12, 3),
-                      "executed_tflops": round(nel * tc_exec_per_el / (tan32_ms * 1e-3) / 1e12, 3),
-                      "peak": round(peak_tf32, 1), "peak_at_kernel_shape": round(peak_tf32_n96, 1),
-                      "unit": "TFLOP/s",
-                      "frac": round(nel * TAN_ALG_FLOPS / (tan32_ms * 1e-3) / 1e12 / peak_tf32, 4),
-                      "frac_executed_of_shape_peak": round(nel * tc_exec_per_el / (tan32_ms * 1e-3) / 1e12
-                                                           / peak_tf32_n96, 4),
-                      "peak_source": "measured: igab_tc_peak (back-to-back tcgen05.mma kind::tf32, M128 x N256 / "
-                                     "N96, one CTA per SM)"}
+    achieved32 = nel * TAN_EXEC_FLOPS / (tan32_ms * 1e-3) / 1e12
+    roofline_mixed = {"bound": "tensor", "pipe": roofline["pipe"], "kernel": "k_tan_sf<float, 1>",
+                      "avg_launch_ms": round(tan32_ms / nl32, 3), "achieved": round(achieved32, 3),
+                      "peak": round(peak64, 3), "unit": "TFLOP/s", "frac": round(achieved32 / peak64, 4),
+                      "flops_definition": roofline["flops_definition"], "peak_source": roofline["peak_source"]}
 
     line = {"metric": METRIC, "value": round(t64 / world, 3), "unit": "ms", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": round(t64, 3), "higher_is_better": False, "scaling": "weak",

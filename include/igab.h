@@ -208,8 +208,8 @@ typedef struct {
 int igab_autotune(igab_ctx *ctx, const double *U_dev, int what, int reps, igab_tune_result *out);
 
 /* ---- batched assembly: many independent meshes of uneven size, each with its own
- * material constants and boundary tables, assembled by one persistent launch per
- * operator (no reference counterpart: the reference runs one mesh per process; each
+ * material constants and boundary tables, assembled by one persistent launch (residual)
+ * or one launch per colour (tangent) over all instances (no reference counterpart: the reference runs one mesh per process; each
  * instance's result is the single-mesh result of igab_residual_device /
  * igab_tangent_device bit for bit).  phys/ge only; Neumann tractions are zero.
  * Instance i owns U/R[dof_offsets[i] .. dof_offsets[i+1]) and
@@ -248,7 +248,7 @@ int igab_batch_last_launch_count(const igab_batch *b, int *n);
 /* one Newton iteration's assembly (residual then tangent) captured in a CUDA graph */
 int igab_batch_graph_capture(igab_batch *b, const double *U_dev, double *R_dev, void *vals_dev, int prec);
 int igab_batch_graph_launch(igab_batch *b);
-/* autotuner of the batch schedule: CTAs per SM of each persistent kernel and the
+/* autotuner of the batch schedule: CTAs per SM of the persistent residual and the
  * instance order (what: bit 0 residual, bit 1 FP64 tangent, bit 2 FP32 tangent), and with
  * bit 3 the colour order (on the sum of the selected kernels, all three when none);
  * the fastest schedule is left applied. */
