@@ -789,7 +789,7 @@ def run_ours(args):
                 "flops_definition": "executed on the tensor path per element (%d: sum-factorised contraction; a dense "
                                     "B^T D B, 64*2*(30*81*10+81*81*10) = %d, is not formed)" % (TAN_EXEC_FLOPS,
                                                                                                TAN_ALG_FLOPS),
-                "dense_equivalent_tflops": round(dense, 3),
+                "executed_tflops": round(achieved, 3), "dense_equivalent_tflops": round(dense, 3),
                 "peak_fp64_fma": round(peak64_fma, 3), "peak_fp64_dmma": round(peak64_dmma, 3),
                 "executed_frac_of_dmma_peak": round(achieved / peak64_dmma, 4),
                 "peak_source": "measured, burst: the larger of the FP64 FMA probe (igab_fma_peak) and the FP64 "
@@ -802,6 +802,7 @@ def run_ours(args):
     achieved32 = nel * TAN_EXEC_FLOPS / (tan32_ms * 1e-3) / 1e12
     roofline_mixed = {"bound": "tensor", "pipe": roofline["pipe"], "kernel": "k_tan_sf<float, 1>",
                       "avg_launch_ms": round(tan32_ms / nl32, 3), "achieved": round(achieved32, 3),
+                      "executed_tflops": round(achieved32, 3),
                       "peak": round(peak64, 3), "unit": "TFLOP/s", "frac": round(achieved32 / peak64, 4),
                       "flops_definition": roofline["flops_definition"], "peak_source": roofline["peak_source"]}
 

@@ -40,8 +40,8 @@
  * version).  Every dot product is a fixed-order reduction: solves are bitwise repeatable.
  *
  * On meshes of some ten thousand dofs a solve is bound by the number of its short kernels, not by their bytes: the
- * smoother's vector updates ride on its products (9 kernels per level and V-cycle instead of 30, 6 products instead of
- * 7), the V-cycle is one graph launch, and a Gram-Schmidt step keeps its coefficients on the device and is read once.
+ * smoother's vector updates ride on its products (at degree 3, 9 kernels per level and V-cycle instead of 30, 6 products
+ * instead of 7), the V-cycle is one graph launch, and a Gram-Schmidt step keeps its coefficients on the device and is read once.
  * 16^3, 108 GMRES iterations of three Newton steps: 50.4 -> 18.9 ms (465 -> 175 us per iteration), and 18.9 -> 13.7 ms
  * (127 us) with the next kernel launched and its matrix rows and tables loaded under the one before (mg_launch), the
  * Gram-Schmidt products of all vectors side by side, and blocks for the dofs there are (8^3: 6.5 -> 4.6 ms, 32^3, 185
