@@ -349,9 +349,9 @@ static int is_capturing(cudaStream_t s, bool *yes)
 
 int igab_scratch_order(igab_ctx *c)
 {
-    if (c->scratch_ev && c->scratch_stream != c->stream)
-        IGAB_CUDA_TRY(cudaStreamWaitEvent(c->stream, c->scratch_ev, 0));
-    c->scratch_stream = c->stream;
+    /* without a look at the stream's handle: equal handles can be two streams (cudaStreamPerThread of two threads, a
+     * stream made after another one was destroyed) */
+    if (c->scratch_ev) IGAB_CUDA_TRY(cudaStreamWaitEvent(c->stream, c->scratch_ev, 0));
     return 0;
 }
 
@@ -360,7 +360,6 @@ int igab_scratch_used(igab_ctx *c)
     if (c->own_capture || (!c->d_scratch[0] && !c->d_scratch[1])) return 0;
     if (!c->scratch_ev) IGAB_CUDA_TRY(cudaEventCreateWithFlags(&c->scratch_ev, cudaEventDisableTiming));
     IGAB_CUDA_TRY(cudaEventRecord(c->scratch_ev, c->stream));
-    c->scratch_stream = c->stream;
     return 0;
 }
 

@@ -164,8 +164,7 @@ struct igab_ctx {
 
     /* scratch of the assembly (igab_scratch) */
     double *d_scratch[2] = {nullptr, nullptr};
-    cudaEvent_t scratch_ev = nullptr;      /* after its last use, on scratch_stream */
-    cudaStream_t scratch_stream = nullptr;
+    cudaEvent_t scratch_ev = nullptr;      /* after its last use */
     bool own_capture = false;              /* the context itself captures its stream */
 
     /* captured assembly graph */
@@ -254,7 +253,7 @@ int igab_launch_tan_getime_level(igab_ctx *c, const double *dU, void *dv, int pr
                                  bool zero);
 /* Scratch arrays of the assembly (igab_capi.cu), allocated on first use and kept by the context.  *out stays null
  * (the caller takes its stateless path) when there is no memory, or while somebody else captures the stream: such
- * a graph could be replayed beside other work of the context.  Uses on different streams are ordered by an event
+ * a graph could be replayed beside other work of the context.  Each use waits for the one before by an event
  * that igab_scratch_used records; igab_scratch_order is the wait alone, before a graph replay. */
 enum igab_scratch_kind { IGAB_SCRATCH_TAN = 0, IGAB_SCRATCH_RES = 1 };
 int igab_scratch(igab_ctx *c, int kind, size_t bytes, double **out);

@@ -1,0 +1,55 @@
+"""The scratch arrays of the assembly beside other contexts, streams and captures."""
+import threading
+
+import numpy as np
+import pytest
+
+from igap4standard_b200 import mesh
+
+pytestmark = pytest.mark.gpu
+
+
+def _mesh(n=16):
+    from igap4standard_b200 import Assembly
+    ne = (n, n, n)
+    return Assembly(ne, mesh.knots_for(ne, perturb=0.1, seed=3), mesh.par_mat_from_lame(1.0, 1.0, 0.1),
+                    *mesh.bc_config0())
+
+
+def _vectors(A, amp=1e-2, seed=1):
+    import torch
+    U = torch.as_tensor(np.random.default_rng(seed).uniform(-amp, amp, A.ndof)).cuda()
+    return U, torch.empty_like(U), torch.empty(A.nnz, dtype=torch.float64, device="cuda")
+
+
+def test_per_thread_stream_of_two_threads(built):
+    """cudaStreamPerThread is one handle and a stream per thread: the second thread's assembly comes after the first
+    one's, with which it shares the scratch, although the handles are equal."""
+    import torch
+    A = _mesh(6)
+    U, R, V = _vectors(A)
+    V2 = torch.empty_like(V)
+    A.tangent_device(U.data_ptr(), V.data_ptr())
+    A.sync()
+    want = V.clone()
+    torch.cuda.synchronize()
+    per_thread = 2
+    A.set_stream(per_thread)
+    done = [None, None]
+
+    def go(i, out, cycles):
+        with torch.cuda.stream(torch.cuda.ExternalStream(per_thread)):
+            if cycles:
+                torch.cuda._sleep(cycles)
+            A.tangent_device(U.data_ptr(), out.data_ptr())
+            done[i] = torch.cuda.Event()
+            done[i].record()
+
+    go(0, V, 400_000_000)          # 0.2 s ahead of the first assembly
+    t = threading.Thread(target=go, args=(1, V2, 0))
+    t.start()
+    t.join()
+    done[1].synchronize()
+    assert done[0].query()
+    torch.cuda.synchronize()
+    assert torch.equal(V, want) and torch.equal(V2, want)
