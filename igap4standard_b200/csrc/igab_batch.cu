@@ -27,6 +27,7 @@
  */
 #include <algorithm>
 #include <numeric>
+#include <utility>
 #include <vector>
 #include <cuda_runtime.h>
 #include "igab_device.cuh"
@@ -61,6 +62,7 @@ struct igab_batch {
     int tan_first[8] = {}, tan_count[8] = {};   /* the tangent's items (behind the residual's nitems) by colour position */
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graph_exec = nullptr;
+    struct { const double *U; double *R; void *vals; int prec; } captured = {};   /* the graph's arguments */
 };
 
 namespace {
@@ -251,6 +253,34 @@ int launch_tangent(igab_batch *b, const double *dU, void *dv, int prec)
     return 0;
 }
 
+/* residual and tangent of the captured arguments as the batch's graph, captured on stream st */
+int capture(igab_batch *b, cudaStream_t st)
+{
+    if (b->graph_exec) { cudaGraphExecDestroy(b->graph_exec); b->graph_exec = nullptr; }
+    if (b->graph) { cudaGraphDestroy(b->graph); b->graph = nullptr; }
+    /* the launchers query occupancy and set kernel attributes: do that once before capture */
+    int g0 = 0, rc = grid_of(b, &g0);
+    if (rc) return rc;
+    IGAB_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+    std::swap(b->stream, st);
+    rc = launch_residual(b, b->captured.U, b->captured.R);
+    if (!rc) rc = launch_tangent(b, b->captured.U, b->captured.vals, b->captured.prec);
+    std::swap(b->stream, st);
+    cudaGraph_t gr = nullptr;
+    cudaError_t e = cudaStreamEndCapture(st, &gr);
+    if (rc) {
+        if (gr) cudaGraphDestroy(gr);
+        return rc;
+    }
+    if (e != cudaSuccess) {
+        igab_set_error("igab_batch_graph_capture: %s", cudaGetErrorString(e));
+        return IGAB_ERR_CUDA;
+    }
+    b->graph = gr;
+    IGAB_CUDA_TRY(cudaGraphInstantiate(&b->graph_exec, b->graph, 0));
+    return 0;
+}
+
 int check_batch_status(igab_batch *b)
 {
     int st = 0;
@@ -417,7 +447,16 @@ extern "C" int igab_batch_set_colour_order(igab_batch *b, int colour_order)
     IGAB_CUDA_TRY(cudaStreamSynchronize(b->stream));
     if (colour_order != b->colour_order) {
         b->colour_order = colour_order;
-        return build_items(b);
+        int rc = build_items(b);
+        /* a captured tangent holds the tiles per colour position, which change with the order: captured anew, on a
+         * stream of its own, as the batch's may be one that cannot be captured */
+        if (!rc && b->graph_exec) {
+            cudaStream_t st = nullptr;
+            IGAB_CUDA_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+            rc = capture(b, st);
+            cudaStreamDestroy(st);
+        }
+        return rc;
     }
     return 0;
 }
@@ -484,27 +523,8 @@ extern "C" int igab_batch_graph_capture(igab_batch *b, const double *U_dev, doub
     BATCH_CHECK(b && U_dev && R_dev && vals_dev, "igab_batch_graph_capture: null argument");
     BATCH_CHECK(prec == IGAB_PREC_FP64 || prec == IGAB_PREC_FP32, "igab_batch_graph_capture: bad precision");
     IGAB_CUDA_TRY(cudaSetDevice(b->device));
-    if (b->graph_exec) { cudaGraphExecDestroy(b->graph_exec); b->graph_exec = nullptr; }
-    if (b->graph) { cudaGraphDestroy(b->graph); b->graph = nullptr; }
-    /* the launchers query occupancy and set kernel attributes: do that once before capture */
-    int g0 = 0, rc = grid_of(b, &g0);
-    if (rc) return rc;
-    IGAB_CUDA_TRY(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-    rc = launch_residual(b, U_dev, R_dev);
-    if (!rc) rc = launch_tangent(b, U_dev, vals_dev, prec);
-    cudaGraph_t gr = nullptr;
-    cudaError_t e = cudaStreamEndCapture(b->stream, &gr);
-    if (rc) {
-        if (gr) cudaGraphDestroy(gr);
-        return rc;
-    }
-    if (e != cudaSuccess) {
-        igab_set_error("igab_batch_graph_capture: %s", cudaGetErrorString(e));
-        return IGAB_ERR_CUDA;
-    }
-    b->graph = gr;
-    IGAB_CUDA_TRY(cudaGraphInstantiate(&b->graph_exec, b->graph, 0));
-    return 0;
+    b->captured = {U_dev, R_dev, vals_dev, prec};
+    return capture(b, b->stream);
 }
 
 extern "C" int igab_batch_graph_launch(igab_batch *b)
