@@ -363,6 +363,18 @@ int igab_scratch_used(igab_ctx *c)
     return 0;
 }
 
+/* cudaMalloc although another stream, of the caller's, may be captured: in the default mode a capture in the global
+ * mode forbids it and is spoilt by it */
+static cudaError_t malloc_beside_captures(double **p, size_t bytes)
+{
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaError_t e = cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) return e;
+    e = cudaMalloc((void **)p, bytes);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    return e;
+}
+
 int igab_scratch(igab_ctx *c, int kind, size_t bytes, double **out)
 {
     *out = nullptr;
@@ -372,7 +384,7 @@ int igab_scratch(igab_ctx *c, int kind, size_t bytes, double **out)
     if (cap && !c->own_capture) return 0;
     if (!c->d_scratch[kind]) {
         if (cap) return 0;
-        if (cudaMalloc((void **)&c->d_scratch[kind], bytes) != cudaSuccess) {
+        if (malloc_beside_captures(&c->d_scratch[kind], bytes) != cudaSuccess) {
             cudaGetLastError();
             c->d_scratch[kind] = nullptr;
             return 0;

@@ -22,6 +22,31 @@ def _vectors(A, amp=1e-2, seed=1):
     return U, torch.empty_like(U), torch.empty(A.nnz, dtype=torch.float64, device="cuda")
 
 
+def test_first_call_beside_a_capture(built):
+    """A context's first assembly, on its own stream, while another stream is captured in the global mode: the capture
+    goes on, and both results are right."""
+    import torch
+    A, B = _mesh(6), _mesh(6)
+    U, R, V = _vectors(A)
+    R1, V1 = torch.empty_like(R), torch.empty_like(V)
+    x = torch.ones(1000, device="cuda")
+    B.residual_device(U.data_ptr(), R1.data_ptr())
+    B.tangent_device(U.data_ptr(), V1.data_ptr())
+    B.sync()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=torch.cuda.Stream(), capture_error_mode="global"):
+        x.add_(1.0)
+        A.residual_device(U.data_ptr(), R.data_ptr())
+        A.tangent_device(U.data_ptr(), V.data_ptr())
+        x.mul_(2.0)
+    A.sync()
+    assert torch.equal(R, R1) and torch.equal(V, V1)
+    g.replay()
+    torch.cuda.synchronize()
+    assert bool((x == 4.0).all())
+
+
 def test_per_thread_stream_of_two_threads(built):
     """cudaStreamPerThread is one handle and a stream per thread: the second thread's assembly comes after the first
     one's, with which it shares the scratch, although the handles are equal."""
