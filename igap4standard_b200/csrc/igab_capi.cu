@@ -8,6 +8,7 @@
 #include <stdio.h>
 #include <string.h>
 #include <algorithm>
+#include <atomic>
 #include <vector>
 #include "igab_internal.h"
 
@@ -363,6 +364,12 @@ int igab_scratch_used(igab_ctx *c)
     return 0;
 }
 
+/* A context of a 16^3 mesh has 146 MB of scratch, three times its matrix, until it is destroyed.  All contexts of a
+ * device together take 4 GB at most; the ones beyond that work without (16^3: 1,096 us instead of 493, 8^3: 1,079
+ * instead of 80), and take theirs when others have given it back. */
+#define SCRATCH_TOTAL ((size_t)4 << 30)
+static std::atomic<size_t> scratch_total[64];
+
 /* cudaMalloc although another stream, of the caller's, may be captured: in the default mode a capture in the global
  * mode forbids it and is spoilt by it */
 static cudaError_t malloc_beside_captures(double **p, size_t bytes)
@@ -384,11 +391,15 @@ int igab_scratch(igab_ctx *c, int kind, size_t bytes, double **out)
     if (cap && !c->own_capture) return 0;
     if (!c->d_scratch[kind]) {
         if (cap) return 0;
-        if (malloc_beside_captures(&c->d_scratch[kind], bytes) != cudaSuccess) {
+        std::atomic<size_t> &total = scratch_total[c->device % 64];
+        if (total.fetch_add(bytes) + bytes > SCRATCH_TOTAL ||
+            malloc_beside_captures(&c->d_scratch[kind], bytes) != cudaSuccess) {
+            total -= bytes;
             cudaGetLastError();
             c->d_scratch[kind] = nullptr;
             return 0;
         }
+        c->scratch_bytes[kind] = bytes;
     }
     if (!cap && (rc = igab_scratch_order(c))) return rc;
     *out = c->d_scratch[kind];
@@ -397,9 +408,11 @@ int igab_scratch(igab_ctx *c, int kind, size_t bytes, double **out)
 
 void igab_scratch_free(igab_ctx *c)
 {
-    for (double *&p : c->d_scratch) {
-        cudaFree(p);
-        p = nullptr;
+    for (int k = 0; k < 2; k++) {
+        cudaFree(c->d_scratch[k]);
+        c->d_scratch[k] = nullptr;
+        scratch_total[c->device % 64] -= c->scratch_bytes[k];
+        c->scratch_bytes[k] = 0;
     }
 }
 

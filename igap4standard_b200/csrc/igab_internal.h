@@ -164,6 +164,7 @@ struct igab_ctx {
 
     /* scratch of the assembly (igab_scratch) */
     double *d_scratch[2] = {nullptr, nullptr};
+    size_t scratch_bytes[2] = {0, 0};
     cudaEvent_t scratch_ev = nullptr;      /* after its last use */
     bool own_capture = false;              /* the context itself captures its stream */
 
@@ -252,9 +253,9 @@ int igab_launch_zero_csr_rows(igab_ctx *c, void *dv, int prec);
 int igab_launch_tan_getime_level(igab_ctx *c, const double *dU, void *dv, int prec, int level, int tx0, int tx1,
                                  bool zero);
 /* Scratch arrays of the assembly (igab_capi.cu), allocated on first use and kept by the context.  *out stays null
- * (the caller takes its stateless path) when there is no memory, or while somebody else captures the stream: such
- * a graph could be replayed beside other work of the context.  Each use waits for the one before by an event
- * that igab_scratch_used records; igab_scratch_order is the wait alone, before a graph replay. */
+ * (the caller takes its stateless path) when there is no memory or the device's share is taken, or while somebody
+ * else captures the stream: such a graph could be replayed beside other work of the context.  Each use waits for the
+ * one before by an event that igab_scratch_used records; igab_scratch_order is the wait alone, before a graph replay. */
 enum igab_scratch_kind { IGAB_SCRATCH_TAN = 0, IGAB_SCRATCH_RES = 1 };
 int igab_scratch(igab_ctx *c, int kind, size_t bytes, double **out);
 int igab_scratch_used(igab_ctx *c);

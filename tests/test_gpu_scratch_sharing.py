@@ -8,6 +8,8 @@ from igap4standard_b200 import mesh
 
 pytestmark = pytest.mark.gpu
 
+TOTAL = 4 << 30        # bytes that the scratch arrays of all contexts of a device take together, at most
+
 
 def _mesh(n=16):
     from igap4standard_b200 import Assembly
@@ -20,6 +22,38 @@ def _vectors(A, amp=1e-2, seed=1):
     import torch
     U = torch.as_tensor(np.random.default_rng(seed).uniform(-amp, amp, A.ndof)).cuda()
     return U, torch.empty_like(U), torch.empty(A.nnz, dtype=torch.float64, device="cuda")
+
+
+def test_scratch_of_many_contexts_is_bounded(built):
+    """36 meshes of 16^3 would take 5.2 GB.  The ones beyond the bound work without a scratch, with the same values, and
+    the scratch of a destroyed context is there for the next one."""
+    import torch
+    many = [_mesh() for _ in range(36)]
+    U, R, V = _vectors(many[0])
+    R1, V1 = torch.empty_like(R), torch.empty_like(V)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    for k, A in enumerate(many):
+        r, v = (R, V) if k else (R1, V1)
+        r.fill_(float("nan")), v.fill_(float("nan"))
+        torch.cuda.synchronize()
+        A.residual_device(U.data_ptr(), r.data_ptr())
+        A.tangent_device(U.data_ptr(), v.data_ptr())
+        A.sync()
+        assert torch.equal(r, R1) and torch.equal(v, V1)
+    torch.cuda.synchronize()
+    grown = free - torch.cuda.mem_get_info()[0]
+    print("%.2f GB" % (grown / 1e9))
+    assert grown <= TOTAL + (256 << 20)          # the comparisons' and the kernels' own memory beside the scratch
+    for A in many:
+        A.close()
+    A = _mesh()
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    A.tangent_device(U.data_ptr(), V.data_ptr())
+    A.sync()
+    assert free - torch.cuda.mem_get_info()[0] >= 16 ** 3 * 4374 * 8
+    assert torch.equal(V, V1)
 
 
 def test_first_call_beside_a_capture(built):
