@@ -913,8 +913,11 @@ extern "C" int igab_history_jacobian_device(igab_ctx *ctx, const double *U_dev, 
     ARG_CHECK(prec == IGAB_PREC_FP64 || prec == IGAB_PREC_FP32, "igab_history_jacobian_device: bad precision");
     IGAB_CUDA_TRY(cudaSetDevice(ctx->device));
     ctx->last_launches = 0;
+    const bool prof = ctx->profiling;
+    ctx->profiling = false;   /* the events are the last residual's and tangent's */
     int rc = igab_launch_tan_getime_level(ctx, U_dev, vals_dev, prec, level, 0, (ctx->ne[0] + 1) / 2, true);
     if (!rc) rc = igab_launch_zero_csr_rows(ctx, vals_dev, prec);
+    ctx->profiling = prof;
     return rc;
 }
 
