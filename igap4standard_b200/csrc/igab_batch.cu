@@ -287,8 +287,7 @@ int check_batch_status(igab_batch *b)
     IGAB_CUDA_TRY(cudaMemcpy(&st, b->d_status, sizeof(int), cudaMemcpyDeviceToHost));
     if (st) {
         IGAB_CUDA_TRY(cudaMemset(b->d_status, 0, sizeof(int)));
-        igab_set_error("batched assembly: a bounded wait gave up (status %d: 1 tensor-core completion, "
-                       "2 colour dependency)", st);
+        igab_set_error("batched assembly: a bounded wait for an earlier colour gave up (status %d)", st);
         return IGAB_ERR_CUDA;
     }
     return 0;

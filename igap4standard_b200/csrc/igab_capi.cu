@@ -425,7 +425,7 @@ static void free_ctx(igab_ctx *c)
     cudaFree(c->d_hval); cudaFree(c->d_neu_row); cudaFree(c->d_neu_ptr); cudaFree(c->d_neu_ent);
     cudaFree(c->d_dnz); cudaFree(c->d_combo_info); cudaFree(c->d_hist);
     cudaFree(c->d_U); cudaFree(c->d_R); cudaFree(c->d_vals);
-    cudaFree(c->d_escale); cudaFree(c->d_lam); cudaFree(c->d_status);
+    cudaFree(c->d_escale); cudaFree(c->d_lam);
     cudaFree(c->d_dens_part); cudaFree(c->d_HH);
     igab_scratch_free(c);
     if (c->scratch_ev) cudaEventDestroy(c->scratch_ev);
@@ -530,8 +530,6 @@ extern "C" int igab_create(const igab_mesh_desc *desc, int device, igab_ctx **ou
             return _e == cudaErrorMemoryAllocation ? IGAB_ERR_NOMEM : IGAB_ERR_CUDA; \
         }                                                                    \
     } while (0)
-    TRY(cudaMalloc((void **)&c->d_status, sizeof(int)));
-    TRY(cudaMemset(c->d_status, 0, sizeof(int)));
     TRY(cudaMalloc((void **)&c->d_rowptr, c->rowptr_h.size() * sizeof(int)));
     TRY(cudaMemcpy(c->d_rowptr, c->rowptr_h.data(), c->rowptr_h.size() * sizeof(int), cudaMemcpyHostToDevice));
 
@@ -852,7 +850,6 @@ extern "C" int igab_tangent(igab_ctx *ctx, const double *U_host, void *vals_host
         if ((rc = igab_launch_check_finite(ctx, ctx->d_vals, nnz, prec, &fin))) return rc;
         IGAB_CUDA_TRY(cudaMemcpyAsync(vals_host, ctx->d_vals, (size_t)nnz * es, cudaMemcpyDeviceToHost, ctx->stream));
         IGAB_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-        if ((rc = igab_check_status(ctx))) return rc;
         if (!fin) { igab_set_error("igab_tangent: non-finite entry"); return IGAB_ERR_NONFINITE; }
         return 0;
     }
@@ -881,8 +878,6 @@ extern "C" int igab_tangent(igab_ctx *ctx, const double *U_host, void *vals_host
     if (rc) return rc;
     IGAB_CUDA_TRY(ce);
     IGAB_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    rc = igab_check_status(ctx);
-    if (rc) return rc;
     if (!fin) { igab_set_error("igab_tangent: non-finite entry"); return IGAB_ERR_NONFINITE; }
     return 0;
 }
@@ -1034,25 +1029,12 @@ extern "C" int igab_set_stream(igab_ctx *ctx, void *cuda_stream)
     return 0;
 }
 
-/* after a stream synchronisation: report (and clear) a kernel's bounded-wait failure */
-int igab_check_status(igab_ctx *ctx)
-{
-    int st = 0;
-    IGAB_CUDA_TRY(cudaMemcpy(&st, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost));
-    if (st) {
-        IGAB_CUDA_TRY(cudaMemset(ctx->d_status, 0, sizeof(int)));
-        igab_set_error("tensor-core tangent kernel: a completion wait gave up (status %d)", st);
-        return IGAB_ERR_CUDA;
-    }
-    return 0;
-}
-
 extern "C" int igab_sync(igab_ctx *ctx)
 {
     ARG_CHECK(ctx, "igab_sync: null context");
     IGAB_CUDA_TRY(cudaSetDevice(ctx->device));
     IGAB_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    return igab_check_status(ctx);
+    return 0;
 }
 
 extern "C" int igab_check_finite(igab_ctx *ctx, const void *dev, long n, int prec, int *all_finite)
@@ -1068,7 +1050,6 @@ extern "C" int igab_set_tile(igab_ctx *ctx, int residual_tile, int tangent_tile)
     ARG_CHECK(residual_tile == 0 || residual_tile == 2 || residual_tile == 4, "igab_set_tile: residual tile must be 2 or 4");
     ARG_CHECK(tangent_tile == 0 || tangent_tile == 2, "igab_set_tile: tangent tile must be 2");
     ctx->tile_res = residual_tile ? residual_tile : 2;
-    ctx->tile_tan = tangent_tile ? tangent_tile : 2;
     ctx->sched_version++;
     return 0;
 }

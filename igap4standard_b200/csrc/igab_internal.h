@@ -114,11 +114,10 @@ struct igab_ctx {
     void *d_vals = nullptr;
     int vals_prec = -1;
 
-    int tile_res = 2, tile_tan = 2;
+    int tile_res = 2;
     int tan_kernel = 1;   /* FP64 tangent: 1 sum factorisation (mma f64), 0 direct SIMT form */
     int tan32_kernel = 1; /* FP32 tangent: 1 the same, FP32 values, 0 direct SIMT form */
     int colour_order = 0; /* igab_colour_order */
-    int *d_status = nullptr;   /* device status word: nonzero after a bounded wait gave up */
     int last_launches = 0;
 
     /* profiling events: [0..2] residual (start, after volume, end), [3..5] tangent */
@@ -194,7 +193,6 @@ int igab_krylov_solve(igab_ctx *c, const void *dvals, int prec, const double *db
                       double atol, int maxit, int *iterations, int *converged, double *rnorm, double *bnorm);
 void igab_krylov_release(igab_ctx *c);
 void igab_newton_release(igab_ctx *c);   /* igab_newton.cu */
-int igab_check_status(igab_ctx *c);      /* after a synchronisation: a bounded wait that gave up -> error */
 /* entry points without a periodic form return IGAB_ERR_UNSUPPORTED for such a mesh */
 #define IGAB_NO_PERIODIC(ctx, name)                                                                   \
     do {                                                                                              \

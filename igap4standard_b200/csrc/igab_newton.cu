@@ -374,7 +374,6 @@ extern "C" int igab_newton_solve(igab_ctx *ctx, double *U_dev, const igab_newton
                     igab_set_error("igab_newton_solve: tangent: %s", cudaGetErrorString(e));
                     return IGAB_ERR_CUDA;
                 }
-                rc = igab_check_status(ctx);
             }
             if (rc) return rc;
             k.ntan++;
