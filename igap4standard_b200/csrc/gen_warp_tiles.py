@@ -1,5 +1,6 @@
-"""Writes igab_warp_tiles8.inc: the split of the FP64 tangent's DMMA tiles over
-the 8 consumer warps of the warp-specialised kernel (igab_tangent_dmma.cu).
+"""Writes igab_warp_tiles8.inc: the split of the DMMA tiles of the FP64 tangent's
+rank-12 form over 8 consumer warps.  No kernel includes the table any more (the
+tangent is igab_tangent_sf.cu); tests/test_warp_tiles.py checks it.
 
 Tiles: the 66 upper 8x8 tiles (I <= J) of the 88x88 element matrix
 K = X'^T diag(s) X' (12 k-steps per batch of 4 Gauss points) and the 10 upper
