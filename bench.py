@@ -273,7 +273,7 @@ class ClockSampler:
 def bench_batch(args, dev, device, barrier):
     """The 512-instance static workload (n^3 elements, n uniform 6..24, own material per
     instance): one Newton iteration's assembly (FP64 residual + FP32 tangent) through the
-    persistent batched launch with the autotuned schedule, and the same work as one
+    batched launches with the autotuned schedule, and the same work as one
     single-mesh assembly per instance for comparison."""
     import ctypes
     import torch

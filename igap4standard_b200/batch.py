@@ -1,6 +1,6 @@
 """Python face of the batched assembly (igab_batch_* of include/igab.h): many
 independent phys/ge meshes of uneven size assembled by one persistent launch
-per operator."""
+(residual) or one launch per colour (tangent) over all of them."""
 import ctypes
 
 import numpy as np

@@ -41,7 +41,8 @@ struct igab_geom {
     double tmass;
 };
 
-/* Batched assembly: the work list of a persistent launch over many meshes.
+/* Batched assembly: the work list of the launches over many meshes (residual: one persistent launch; tangent: one
+ * launch per sweep position, in which the wait below finds its counts complete).
  * item = (instance, sweep position p, tile, colour), ordered colour-major in the
  * batch's colour order (colour = igab_colour_at(order, p)); done[8 i + p] counts the
  * finished tiles of position p of instance i, need[8 i + p] how many there are.  A

@@ -4,8 +4,8 @@
  * Schedule (both operators): the mesh is cut into tiles of TE^3 elements
  * (TE >= 2).  Tiles are coloured by the parity of their tile coordinates
  * (8 colours); two tiles of one colour are at least TE elements apart, so
- * the control points they touch are disjoint and one launch per colour can
- * read-modify-write the global residual / CSR values without atomics.  Inside
+ * the control points they touch are disjoint and one launch per colour adds to
+ * the global residual / CSR values without two tiles meeting at an entry.  Inside
  * a tile the accumulation order is fixed, so results are bitwise repeatable.
  *
  * Residual (src/snesiga_Residual.c:99-174): per element, 64 threads, one per

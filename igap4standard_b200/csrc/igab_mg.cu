@@ -23,7 +23,7 @@
  * prolonged corrections, which keeps the V-cycle symmetric.
  *
  * Smoother: Chebyshev polynomial of degree 6 in D^-1 K on [1.1 lmax / 100, 1.1 lmax], lmax
- * estimated by power iteration; the same polynomial before and after the coarse
+ * by 40 power iterations; the same polynomial before and after the coarse
  * correction, so the V-cycle is a symmetric preconditioner and CG applies.
  *
  * Coarsest level: its tangent (symmetric positive definite: the zero-state tangent with
@@ -39,16 +39,18 @@
  * boundary tables' values or the element scales change (the context's parameter
  * version).  Every dot product is a fixed-order reduction: solves are bitwise repeatable.
  *
- * On meshes of some ten thousand dofs a solve is bound by the number of its short kernels, not by their bytes: the
- * smoother's vector updates ride on its products (at degree 3, 9 kernels per level and V-cycle instead of 30, 6 products
- * instead of 7), the V-cycle is one graph launch, and a Gram-Schmidt step keeps its coefficients on the device and is read once.
- * 16^3, 108 GMRES iterations of three Newton steps: 50.4 -> 18.9 ms (465 -> 175 us per iteration), and 18.9 -> 13.7 ms
- * (127 us) with the next kernel launched and its matrix rows and tables loaded under the one before (mg_launch), the
- * Gram-Schmidt products of all vectors side by side, and blocks for the dofs there are (8^3: 6.5 -> 4.6 ms, 32^3, 185
- * iterations: 110.5 -> 95.2 ms).  What is left at 16^3 is 7 fine products of 9 us (6 us of them latency: three passes
- * of loads on 1.2 waves of blocks) and some 25 other kernels of 3-5 us (with the smoother's degree 3 of that time; now
- * 6, and 45 iterations of 200 us).  Left out: more blocks per SM by fewer
- * registers (spills, 14.0-19.6 ms), rows cut at whole runs of columns (half the instructions, no faster, 32^3 101.6).
+ * On meshes of some ten thousand dofs a solve is bound by the number of its short kernels, not by their bytes.  The
+ * smoother's vector updates ride on its products: a level but the coarsest takes 12 products and two transfers per
+ * V-cycle.  The V-cycle is one graph launch, a Gram-Schmidt step keeps its coefficients on the device and is read once,
+ * each kernel is launched, and its matrix rows and tables loaded, under the one before (mg_launch), the Gram-Schmidt
+ * products of all vectors run side by side, and a kernel has blocks for the dofs there are.  GMRES of three Newton steps
+ * at 8^3 / 16^3 / 24^3 / 32^3: 3.1 / 9.4 / 28.1 / 70.6 ms, 30 / 47 / 63 / 80 iterations of 104 / 199 / 446 / 883 us.
+ * What is left at 16^3 are 12 fine products of 9 us (6 us of them latency: three passes of loads on 1.2 waves of blocks)
+ * and some 26 other kernels of 3-5 us.
+ * The parts of it, measured at degree 3 (6 products per level) at 16^3: fused updates, graph and device coefficients
+ * 465 -> 175 us per iteration, launches under one another 175 -> 127 us (8^3: 6.5 -> 4.6 ms, 32^3, 185 iterations:
+ * 110.5 -> 95.2 ms); left out: more blocks per SM by fewer registers (spills, 14.0-19.6 ms against 13.7), rows cut at
+ * whole runs of columns (half the instructions, no faster, 32^3 101.6).
  * Measured and rejected: the smoothing operators stored in half precision (64^3: 4.58 ->
  * 4.36 ms per GMRES iteration, but one more iteration per solve; no gain per Newton step).
  */
@@ -611,7 +613,8 @@ int estimate_lmax(igab_mg *m, mg_level &L)
 
 /* The interval is wide and the degree high, as the operator is of fourth order: an error of half the coarse mesh's
  * resolution has 2^-4 or less of lmax, and the rediscretised coarse operator corrects the modes near that poorly.
- * GMRES of three Newton steps at 8^3 / 16^3 / 32^3 (ms; iterations at 16^3): degree 3, ratio 10: 4.6 / 13.8 / 95.2
+ * GMRES of three Newton steps at 8^3 / 16^3 / 32^3 (ms; iterations at 16^3; lmax of 12 power iterations, 4% lower than
+ * now at 16^3): degree 3, ratio 10: 4.6 / 13.8 / 95.2
  * (108); degree 3, ratio 30: 16^3 11.7, 32^3 79.7 (91); degree 4, 30: 11.0, 78.6 (73); degree 6: ratio 40 10.4, 80.2,
  * 80 2.8 / 9.3 / 70.7 (47), 120 3.3 / 8.7 / 68.2 (44), 200 4.1 / 8.9 / 64.6; degree 8: ratio 100 2.8 / 8.7 / 71.7 (35),
  * 200 3.7 / 8.6 / 65.1; degree 10, 200: 3.5 / 8.8 / 67.4; degree 2, 10: 15.0, 92.2 (140).

@@ -33,9 +33,10 @@
  * the value components; the additional work is in the point matrices only.  FP64 throughout; FP32 values round
  * at the store.
  *
- * Measured (tangent alone).  64^3: 20.5 ms, FP64 and FP32 values, against 96.6 ms for the rank-12 form on the
- * same pipe and 40.4 ms for its TF32 tcgen05 form, whose values had 1.3e-6 error against 64 bits (8e-8 here).
- * 32^3 transient: 6.1 ms against 33.7 ms for the rank-24 form.  Bound by instruction latency in the short
+ * Measured (tangent alone).  64^3: 20.5 ms FP64, 19.9 ms FP32 values, against 96.1 ms for the rank-12 form on the
+ * same pipe and 41.1 ms for its TF32 tcgen05 form.  Error of the FP32 values against FP64, in the norm of all and the
+ * worst entry over its row's largest: 7.6e-8 and 5.4e-7, TF32 form 1.3e-6 and 2.8e-6.  32^3 transient: 4.7 ms against
+ * 35.3 ms for the rank-24 form.  Bound by instruction latency in the short
  * barrier phases (IPC 0.36 per scheduler; tensor and FP64 pipe 47%).  Measured and left out: the second step fed
  * from the first one's accumulators in registers, without T1 (23.0 ms: it moves the third step into the same
  * warps' serial chain); totals by shuffles instead of a product with ones (+0.7 ms); one copy of each part

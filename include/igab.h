@@ -108,9 +108,10 @@ int igab_set_history(igab_ctx *ctx, int level, const double *U, int on_device);
 int igab_residual(igab_ctx *ctx, const double *U_host, double *R_host);
 int igab_residual_device(igab_ctx *ctx, const double *U_dev, double *R_dev);
 /* vals: nnz doubles (IGAB_PREC_FP64) or floats (IGAB_PREC_FP32).  igab_tangent
- * assembles meshes of 23 or more elements along x slab by slab along x and downloads
- * the rows each slab finishes on a second stream while the next slabs are assembled
- * (pinned vals_host overlaps fully); the values are bitwise those of igab_tangent_device. */
+ * assembles in parts along x (some layers of elements at a time, or slabs of tiles where
+ * the layers are large) and downloads the rows each part finishes on a second stream while
+ * the next ones are assembled (pinned vals_host overlaps fully); the values are bitwise
+ * those of igab_tangent_device. */
 int igab_tangent(igab_ctx *ctx, const double *U_host, void *vals_host, int prec);
 int igab_tangent_device(igab_ctx *ctx, const double *U_dev, void *vals_dev, int prec);
 
@@ -158,8 +159,8 @@ int igab_fma_peak(int device, int prec, double *tflops);
 /* FP64 tensor-pipe throughput probe (TFLOP/s): back-to-back mma.sync m8n8k4 f64 on
  * independent accumulators, 32 warps per SM (the pipe of the FP64 tangent's products) */
 int igab_dmma_peak(int device, double *tflops);
-/* Check of a tcgen05 operand layout and its descriptors (no reference counterpart): one CTA computes A B^T for fixed small-integer A (128 x 32) and
- * B (96 x 32) with the M 128 / N 96 and M 128 / N 32 instruction shapes; out (128 x 160 floats,
+/* Check of a tcgen05 operand layout and its descriptors (no reference counterpart): one CTA
+ * computes A B^T for fixed small-integer A (128 x 32) and B (96 x 32) with the M 128 / N 96 and M 128 / N 32 instruction shapes; out (128 x 160 floats,
  * row-major) receives accumulator columns 0-95 (A B^T), 96-127 (A B[0:32]^T) and 128-159
  * (A B[0:32]^T over K 0-15 minus it over K 16-31, the negate-A form). */
 int igab_tc_selftest(int device, float *out);
@@ -209,8 +210,8 @@ int igab_autotune(igab_ctx *ctx, const double *U_dev, int what, int reps, igab_t
 
 /* ---- batched assembly: many independent meshes of uneven size, each with its own
  * material constants and boundary tables, assembled by one persistent launch (residual)
- * or one launch per colour (tangent) over all instances (no reference counterpart: the reference runs one mesh per process; each
- * instance's result is the single-mesh result of igab_residual_device /
+ * or one launch per colour (tangent) over all instances (no reference counterpart: the
+ * reference runs one mesh per process; each instance's result is the single-mesh result of igab_residual_device /
  * igab_tangent_device bit for bit).  phys/ge only; Neumann tractions are zero.
  * Instance i owns U/R[dof_offsets[i] .. dof_offsets[i+1]) and
  * vals[nnz_offsets[i] .. nnz_offsets[i+1]) in its own numbering and AIJ pattern;
@@ -228,7 +229,8 @@ int igab_batch_refresh(igab_batch *b);
 int igab_batch_set_stream(igab_batch *b, void *cuda_stream);
 int igab_batch_set_schedule(igab_batch *b, int ctas_res, int ctas_tan64, int ctas_tan32, int order);
 int igab_batch_get_schedule(const igab_batch *b, int *ctas_res, int *ctas_tan64, int *ctas_tan32, int *order);
-/* colour order of the batch's work list (igab_colour_order; natural by default) */
+/* colour order of the batch's work list (igab_colour_order; natural by default); a captured
+ * graph is captured anew, so that its replays follow */
 int igab_batch_set_colour_order(igab_batch *b, int colour_order);
 int igab_batch_get_colour_order(const igab_batch *b, int *colour_order);
 /* The launches below return once enqueued.  A tile of colour c waits (bounded) for the
