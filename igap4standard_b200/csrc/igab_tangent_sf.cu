@@ -14,8 +14,8 @@
  * against 6.98 MFLOP of the rank-12 form X^T Phi'' X it replaces.
  *
  * Each step is a product W (pairs x 4 points) B (4 points x columns): the 9 pairs (a, b) of a direction
- * are one m8 tile without the pair (1, 1), plus the total sum_q B.  As the three functions sum to 1
- * (and their derivatives to 0), the entry (1, 1) is the total minus the other eight, so the eight rows
+ * are one m8 tile without the pair (1, 1), plus the total sum_q B.  As the three functions sum to 1 (in
+ * the tables that the kernel uses, sf_sum) and their derivatives to 0, the entry (1, 1) is the total minus the other eight, so the eight rows
  * come out as they are, one product serves all nine pairs, and the totals only need the terms without a
  * derivative in that direction (a sum over four lanes).  The totals are carried as row / column 4 through
  * all steps and turned into the entries (1, 1) on the finished element matrix, direction by direction.
@@ -584,11 +584,46 @@ __device__ __forceinline__ void sf_interp_y(sf_smem<NR> &S, int buf, int tid)
         SF_C(S)[o] = By[qy * 9 + ky] * a0[0] + By[qy * 9 + 3 + ky] * a0[9] + By[qy * 9 + 6 + ky] * a0[18];
     }
 }
+/* The basis's denominators carry a guard of 1e-15 (igab_bspline_p2), so the three functions sum to 1 only within 1e-15
+ * over the element's width (their derivatives do sum to 0).  The totals need 1, so the tables are divided by the sum
+ * and the weights multiplied by its square, which leaves the products as they are.  Without it the values were 1e-12
+ * of the row's largest off at 64^3 on the unit cube, and 2e-7 on a cube of 1e-6; now 3e-15.  It costs nothing that
+ * shows (64^3 20.5 ms): both steps run on threads that wait; the totals weighted with the sum's square instead, a
+ * register more in each step, took 2.6%.
+ * The sum of thread i < 12: direction i / 4, point i % 4; an empty element has any sum and no weight. */
+template <int NR>
+__device__ __forceinline__ double sf_sum(const sf_smem<NR> &S, int buf, int i)
+{
+    const double *t = S.tab[buf][i >> 2] + (i & 3) * 9;
+    const double s = t[0] + t[3] + t[6];
+    return s > 1e-3 ? s : 1.0;
+}
+/* beside the last interpolation, which still needs the tables as they are */
+template <int NR>
+__device__ __forceinline__ void sf_norm_weights(sf_smem<NR> &S, int buf, int i)
+{
+    if (i < 0 || i >= 12) return;
+    const double s = sf_sum<NR>(S, buf, i);
+    S.wh[buf][i >> 2][i & 3] *= s * s;
+}
+/* and beside the point data, which does not */
+template <int NR>
+__device__ __forceinline__ void sf_norm_tab(sf_smem<NR> &S, int buf, int i)
+{
+    if (i < 0 || i >= 12) return;
+    const double r = 1.0 / sf_sum<NR>(S, buf, i);
+    double *t = S.tab[buf][i >> 2] + (i & 3) * 9;
+#pragma unroll
+    for (int k = 0; k < 9; k++) t[k] *= r;
+}
 /* F and G of component tid / 64 at point tid % 64; for NR = 2 of the hat fields r00 m + r01 h, r11 h */
 template <int NR>
 __device__ __forceinline__ void sf_interp_x(sf_smem<NR> &S, const igab_geom &g, const sf_coef &R, int buf, int tid)
 {
-    if (tid >= 192) return;
+    if (tid >= 192) {
+        sf_norm_weights<NR>(S, buf, tid - 192);
+        return;
+    }
     using A = pt_at<NR>;
     const int i = tid >> 6, p = tid & 63, qz = p & 3, qy = (p >> 2) & 3, qx = p >> 4;
     const double *Bx = S.tab[buf][0] + qx * 9;
@@ -644,6 +679,7 @@ template <int NR>
 __device__ __forceinline__ void sf_point_data(sf_smem<NR> &S, const igab_geom &g, const sf_coef &R, int buf, int tid)
 {
     using A = pt_at<NR>;
+    sf_norm_tab<NR>(S, buf, tid - 224);
     const int p = tid & 63, qz = p & 3, qy = (p >> 2) & 3, qx = p >> 4;
     double *pt = S.pt + p;
     const double w = S.wh[buf][0][qx] * S.wh[buf][1][qy] * S.wh[buf][2][qz] * S.esc[buf];
